@@ -270,7 +270,8 @@ int gpumhd_tile_from(gpumhd_ctx* ctx, gpumhd_ctx* src);
 
 /* ---- launch shapes (no counterpart in the reference: GPU tiling only) ----
  * stage_zchunk: z planes per stage-kernel block (0: chosen from the GPU's
- * occupancy); tvd_chunk: cells per thread of the y / z TVD sweeps (0: 32).
+ * occupancy); tvd_chunk: cells per thread of the y / z TVD sweeps (0: up to 32,
+ * fewer on boxes that do not fill the GPU).
  * Results do not depend on them. */
 int gpumhd_set_tuning(gpumhd_ctx* ctx, int stage_zchunk, int tvd_chunk);
 /* Test hook of the TMA stage kernel's bounded waits (no counterpart in the

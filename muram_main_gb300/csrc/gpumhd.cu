@@ -66,7 +66,8 @@ struct gpumhd_ctx {
   bool tma = false;
   CUtensorMap mapS[3];
   CUtensorMap mapP[2];
-  // launch shapes of the fused step (0: defaults); set by gpumhd_set_tuning / gpumhd_autotune
+  // launch shapes of the fused step (0: defaults); set by gpumhd_set_tuning /
+  // gpumhd_autotune (tune_td < 0: at most -tune_td cells per thread)
   int tune_zc = 0, tune_td = 0;
   // test hook of the TMA stage kernel's bounded waits (gpumhd_test_tma_wait)
   int tm_withhold_last = 0;
@@ -1792,7 +1793,7 @@ extern "C" int gpumhd_get_tuning(gpumhd_ctx* ctx, int* stage_kernel, int* stage_
   if (!ctx) return GPUMHD_E_INVALID;
   if (stage_kernel) *stage_kernel = (ctx->tma && ctx->p.stage_kernel == 0) ? 0 : 1;
   if (stage_zchunk) *stage_zchunk = ctx->tune_zc;
-  if (tvd_chunk) *tvd_chunk = ctx->tune_td;
+  if (tvd_chunk) *tvd_chunk = ctx->tune_td < 0 ? -ctx->tune_td : ctx->tune_td;
   return GPUMHD_OK;
 }
 
@@ -1904,15 +1905,19 @@ extern "C" int gpumhd_autotune(gpumhd_ctx* ctx, int trial_steps, double* best_ms
   }
   ctx->p.stage_kernel = bk;
   ctx->tune_zc = bz;
+  // the chosen TVD chunk is an upper limit (stored negative): on a box that
+  // does not fill the GPU the launcher's shorter chunks stay in force
   const int tds[] = {32, 16, 64};
+  double best_td = 1e300;
   for (int td : tds) {
     if (rc) break;
-    ctx->tune_td = td;
+    ctx->tune_td = -td;
     double ms = 0.0;
     rc = restore();
     if (!rc) rc = time_steps(ctx, trial_steps, &ms);
-    if (!rc && ms < best) { best = ms; btd = td; }
+    if (!rc && ms < best_td) { best_td = ms; btd = -td; }
   }
+  if (best_td < best) best = best_td;
   ctx->tune_td = btd;
   ctx->p.compensated = sv.comp;
   if (!rc) rc = restore();
@@ -2078,7 +2083,10 @@ extern "C" int gpumhd_ensemble_set_schedule(gpumhd_ensemble* e, int steps_per_it
 // chunks, short TVD chunks: many blocks, each with its own prologue planes and
 // stencil halo); inside an ensemble the other boxes fill it, so longer
 // marches can pay.  Candidates: each box's current shapes, and stage z chunks
-// of half or all of the box's z extent with TVD chunks of 64 or 128 cells;
+// of a half or a quarter of the box's z extent with TVD chunks of 16, 64 or 128
+// cells (20 steps of 16 boxes of 32 to 96 cells a side: 21.9 ms with the boxes'
+// own shapes, 20.2 with quarters and 16; 24.3 with halves and 128, which is the
+// fastest for 64 boxes of up to 128 a side; the whole z extent 28 and more);
 // timed over trial_steps steps of the whole ensemble (branches largest box
 // first) from the boxes' current states, which are restored afterwards.
 extern "C" int gpumhd_ensemble_autotune(gpumhd_ensemble* e, int trial_steps, double* best_ms) {
@@ -2101,13 +2109,13 @@ extern "C" int gpumhd_ensemble_autotune(gpumhd_ensemble* e, int trial_steps, dou
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (rc == 0 && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
     rc = efail(e, GPUMHD_E_CUDA, "ensemble autotune: events");
-  struct Cand { int z; int td; };  // z: 0 = each box's own shapes, 1 = half the z extent, 2 = all of it
-  const Cand cands[] = {{0, 0}, {1, 64}, {1, 128}, {2, 64}, {2, 128}};
+  struct Cand { int z; int td; };  // z: 0 = each box's own shapes, else 1/z of the z extent
+  const Cand cands[] = {{0, 0}, {2, 16}, {4, 16}, {2, 64}, {2, 128}};
   auto apply = [&](const Cand& k) {
     for (size_t b = 0; b < nb; b++) {
       gpumhd_ctx* x = e->box[b];
       const int nz = x->c.g.nz;
-      x->tune_zc = k.z == 0 ? zc0[b] : (k.z == 1 ? std::max(1, nz / 2) : nz);
+      x->tune_zc = k.z == 0 ? zc0[b] : std::max(1, nz / k.z);
       x->tune_td = k.z == 0 ? td0[b] : k.td;
       if (x->graph) { cudaGraphExecDestroy(x->graph); x->graph = nullptr; }
     }

@@ -1,6 +1,8 @@
 // Kernel launchers, instantiated once per state type in its own translation
 // unit (FP64 without FMA contraction, FP32 with it).
 #pragma once
+#include <math.h>
+
 #include "gpumhd_stage_tm.cuh"
 #include "gpumhd_divb.cuh"
 #include "gpumhd_bnd.cuh"
@@ -41,7 +43,7 @@ struct Launch {
   static void stage(const Consts& c, const R* Uin, const R* Pin, const R* U0, R* Uout, R* Pout, R* Res, Dyn* dyn,
                     int stage, bool resid, int write_pres, cudaStream_t s, const CUtensorMap* mu = nullptr,
                     const CUtensorMap* mp = nullptr, int zc = 0, Rem<R>* Cc = nullptr);
-  // td: cells per thread along the y / z sweeps (0: 32); the sweeps store the
+  // td: cells per thread along the y / z sweeps (0: tvd_chunk's choice; negative: that, but at most -td); the sweeps store the
   // interior (and after a first half pass the periodic images), step_finish
   // then ends the step
   // dg (per-routine TVDlimit on an output step): the diagnostics, through the
@@ -105,6 +107,58 @@ inline int grid_for(long long n, int block) {
   return (int)b;
 }
 
+// z planes per stage block (bxy column tiles, nz planes, res resident blocks).
+// A block's time is about its planes plus two (FP64 one) for its prologue (four
+// z-flux planes) per wave of resident blocks; where two blocks share an SM
+// (FP32), a first wave of at most one block per SM takes 0.85 of a full wave's
+// time per plane, and over many waves the last, partly filled one is half
+// hidden.  Small boxes therefore march short chunks, down
+// to one plane (16 x 12 x 8 FP32: 19.2 us per stage with 4 planes, 11.2 with
+// 1; 96^3 FP32: 66 us with 24 planes, 48 with 12), large ones the longest chunks that fill the last wave.  A
+// shorter chunk has to be 1 % better to be taken.
+template <class R>
+inline int stage_chunk(long long bxy, int nz, int res) {
+  const double half = sizeof(R) == 4 ? 0.85 : 1.0, first = sizeof(R) == 4 ? 2.0 : 1.0;
+  int best_zc = nz;
+  double best = 1e300;
+  for (int nzc = 1; nzc <= nz && nzc <= 1024; nzc++) {
+    const int zc = (nz + nzc - 1) / nzc;
+    if (nzc > 1 && (nz + nzc - 2) / (nzc - 1) == zc) continue;  // the same chunks again
+    const double w = (double)(bxy * ((nz + zc - 1) / zc)) / res, cw = ceil(w);
+    const double waves = w <= 0.5 ? half : (cw <= 2.0 ? cw : 0.5 * (w + cw));
+    const double cost = (zc + first) * waves;
+    if (cost < 0.99 * best) { best = cost; best_zc = zc; }
+  }
+  return best_zc;
+}
+
+// Cells per thread of a y / z TVD sweep (pencils: their number, n1: their
+// cells).  A thread's time is about its cells plus four (FP32) or 1.5 (FP64)
+// for the stencil's first cells; per cell a wave of blocks costs a latency part
+// and an issue part that grows with its fill (FP32, fitted: 0.7 + 1.05 w us at
+// w of a full wave), in FP64 the pipe time of its blocks, where blocks of a
+// second wave start in pairs on the SMs that come free.  Measured, y sweep:
+// FP32 16 x 12 x 8 19.4 us with 32 cells, 11.1 with 2; 64^3 34.6 us with 32,
+// 19.0 with 4; 128^3 77 us with 32, 75 with 16; 192 x 128 x 256 179 us with
+// 32, 182 with 16, 198 with 64; FP64 64^3 0.99 ms with 32, 0.51 with 8.
+template <class R>
+inline int tvd_chunk(long long pencils, int n1, int most) {
+  constexpr bool f32 = sizeof(R) == 4;
+  const int per_sm = f32 ? 4 : 2;  // resident blocks of 128 threads
+  int best_td = most;
+  double best = 1e300;
+  for (int td = most; td >= 2; td /= 2) {
+    const long long blocks = (pencils * ((n1 + td - 1) / td) + 127) / 128;
+    const double w = (double)blocks / (152.0 * per_sm), full = floor(w);
+    double waves;
+    if (f32) waves = 1.75 * full + (w > full ? 0.7 + 1.05 * (w - full) : 0.0);
+    else waves = w <= 0.5 ? 0.5 : ceil(w);
+    const double cost = ((td < n1 ? td : n1) + (f32 ? 4.0 : 1.5)) * waves;
+    if (cost < 0.99 * best) { best = cost; best_td = td; }
+  }
+  return best_td;
+}
+
 #ifdef GPUMHD_LAUNCH_IMPL
 template <class R>
 int Launch<R>::stage_smem_bytes() {
@@ -162,22 +216,9 @@ void Launch<R>::stage(const Consts& c, const R* Uin, const R* Pin, const R* U0, 
   const int TX = tma ? StageTileTm<R>::TX : StageTile<R>::TX, TY = tma ? StageTileTm<R>::TY : StageTile<R>::TY;
   const Geom& g = c.g;
   const int bx = (g.nx + TX - 1) / TX, by = (g.ny + TY - 1) / TY;
-  // z chunk length: each block computes 4 extra z-flux planes before its
-  // first output plane, and a partly filled last wave idles the GPU; pick the
-  // chunk count that maximises (useful share of the waves) / (1 + 4/zc).
   const long long bxy = (long long)bx * by;
   const int res0 = tma ? resident_tm_blocks : resident_stage_blocks;
-  const int res = res0 > 0 ? res0 : 304;
-  int zc = g.nz;
-  double best = -1.0;
-  for (int nzc = 1; nzc <= 64 && nzc <= g.nz; nzc++) {
-    const int zcc = (g.nz + nzc - 1) / nzc;
-    if (zcc < 4 && nzc > 1) break;
-    const long long blocks = bxy * ((g.nz + zcc - 1) / zcc);
-    const long long waves = (blocks + res - 1) / res;
-    const double eff = ((double)blocks / (double)(waves * res)) / (1.0 + 4.0 / zcc);
-    if (eff > best + 1e-9) { best = eff; zc = zcc; }
-  }
+  int zc = stage_chunk<R>(bxy, g.nz, res0 > 0 ? res0 : 304);
   if (zc_force > 0) zc = zc_force < g.nz ? zc_force : g.nz;
   const int bz = (g.nz + zc - 1) / zc;
   dim3 grid(bx, by, bz);
@@ -226,7 +267,6 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
   ta.dir = dir;
   ta.mode = mode;
   ta.only_two_half = only_two_half;
-  ta.td = td > 0 ? td : 32;
   const long long sx = 1, sy = g.sx, sz = (long long)g.sx * g.sy;
   // pencil ranges of TVDlimit's three sweeps (src/tvdlimit_SR.C:199-205, 671-672)
   if (dir == 0) {
@@ -242,6 +282,7 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
     ta.nb = g.ny; ta.b0 = GH; ta.sb = sy;
     ta.sd = sz; ta.n1 = g.nz;
   }
+  ta.td = td > 0 ? td : tvd_chunk<R>((long long)ta.na * ta.nb, ta.n1, td < 0 ? -td : 32);
   const long long nch = (ta.n1 + ta.td - 1) / ta.td;
   const long long total = (long long)ta.na * ta.nb * nch;
   const int block = 128;

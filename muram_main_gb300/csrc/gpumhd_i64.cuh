@@ -22,23 +22,22 @@
 // Arguments or results outside the normal range (zeros but for a zero
 // numerator, subnormals, infinities, NaN, logs below 1/16 in size) take the
 // built-in operation, so every result there is what it was.
-// The functions are compiled for the host too, where a test compares them with
-// the host's own operations.
+// Outside nvcc the functions are host code, which a test compares with the
+// host's own operations.
 #pragma once
 #include <stdint.h>
 #include <string.h>
 #ifdef __CUDACC__
-#define I64_FN static __device__ __host__ __forceinline__
-#define I64_COLD static __device__ __host__ __noinline__
+#define I64_FN static __device__ __forceinline__
+#define I64_COLD static __device__ __noinline__
+#define I64_TABLE(ty, name) static __device__ const ty name[128]
+#define I64_AT(t, i) __ldg(&t[i])
 #else
 #include <math.h>
 #define I64_FN static inline
 #define I64_COLD static inline
-#endif
-#ifdef __CUDA_ARCH__
-#define I64_TABLE(ty, name) static __device__ const ty name[128]
-#else
-#define I64_TABLE(ty, name) static const ty name##_h[128]
+#define I64_TABLE(ty, name) static const ty name[128]
+#define I64_AT(t, i) t[i]
 #endif
 
 #ifndef I64_SEED_SKEW
@@ -58,7 +57,7 @@ I64_TABLE(uint32_t, LOG_C) = {
     586, 583, 580, 578, 575, 573, 570, 568, 565, 563, 561, 558, 556, 554, 551, 549,
     547, 544, 542, 540, 538, 535, 533, 531, 529, 527, 525, 523, 521, 519, 517, 515};
 // -ln(c_i / 2^10), Q0.64
-I64_TABLE(uint64_t, LOG_T) = {
+I64_TABLE(unsigned long long, LOG_T) = {
     0x0ull, 0x1c189cbb0e27fabull, 0x3c719c606662177ull, 0x5d0c874f401b4a7ull,
     0x7dea6c59e0a156dull, 0x9ae45fd5098357dull, 0xb8132d2a873bb90ull, 0xd9aeecdac5d5675ull,
     0xf7518e0035c3dd8ull, 0x1152b799bb3cc89bull, 0x1333d7f8183f4b6aull, 0x1518874226130a1eull,
@@ -92,7 +91,7 @@ I64_TABLE(uint64_t, LOG_T) = {
     0xa9157039c51ebe71ull, 0xaa0dae5cbcc048b3ull, 0xab06de228a9e3499ull, 0xac010163639a9787ull,
     0xacfc19fcea147ffaull, 0xadf829d243487034ull, 0xaef532cc2d1a7e8dull, 0xaff336d9144c9071ull};
 // 2^(j/128), Q1.63
-I64_TABLE(uint64_t, EXP_T) = {
+I64_TABLE(unsigned long long, EXP_T) = {
     0x8000000000000000ull, 0x80b1ed4fd999ab6cull, 0x8164d1f3bc030773ull, 0x8218af4373fc25ecull,
     0x82cd8698ac2ba1d7ull, 0x8383594eefb6ee37ull, 0x843a28c3acde4046ull, 0x84f1f656379c1a29ull,
     0x85aac367cc487b15ull, 0x8664915b923fba04ull, 0x871f61969e8d1010ull, 0x87db357ff698d792ull,
@@ -127,7 +126,7 @@ I64_TABLE(uint64_t, EXP_T) = {
     0xfa83b2db722a033aull, 0xfbdfed6ce5f09c49ull, 0xfd3e0c0cf486c175ull, 0xfe9e115c7b8f884cull};
 
 I64_FN uint64_t bits_of(double x) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return (uint64_t)__double_as_longlong(x);
 #else
   uint64_t u;
@@ -136,7 +135,7 @@ I64_FN uint64_t bits_of(double x) {
 #endif
 }
 I64_FN double of_bits(uint64_t u) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return __longlong_as_double((long long)u);
 #else
   double x;
@@ -145,7 +144,7 @@ I64_FN double of_bits(uint64_t u) {
 #endif
 }
 I64_FN uint64_t mulhi(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return __umul64hi(a, b);
 #else
   return (uint64_t)(((unsigned __int128)a * b) >> 64);
@@ -157,14 +156,14 @@ I64_FN uint64_t mul64x32(uint64_t a, uint32_t b) {
   return (uint64_t)(uint32_t)(a >> 32) * b + (((uint64_t)(uint32_t)a * b) >> 32);
 }
 I64_FN int clz64(uint64_t a) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return __clzll((long long)a);
 #else
   return __builtin_clzll(a);
 #endif
 }
 I64_FN float float_of(uint32_t u) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return __uint_as_float(u);
 #else
   float f;
@@ -173,7 +172,7 @@ I64_FN float float_of(uint32_t u) {
 #endif
 }
 I64_FN uint32_t bits32(float f) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   return __float_as_uint(f);
 #else
   uint32_t u;
@@ -183,7 +182,7 @@ I64_FN uint32_t bits32(float f) {
 }
 // seeds, relative error below 2^-21 (a normal)
 I64_FN float rcp_seed(float a) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
@@ -192,7 +191,7 @@ I64_FN float rcp_seed(float a) {
 #endif
 }
 I64_FN float rsqrt_seed(float a) {
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
@@ -215,6 +214,28 @@ I64_FN bool is_nan(double a) { return (bits_of(a) & 0x7fffffffffffffffull) > 0x7
 // fmax, fmin: a NaN yields the other argument
 I64_FN double fmax2(double a, double b) { return (lt(a, b) || is_nan(a)) ? b : a; }
 I64_FN double fmin2(double a, double b) { return (lt(b, a) || is_nan(a)) ? b : a; }
+
+// ------------------------------------------------- exact scaling, conversion
+// x / 2 and x / 4
+I64_FN double half(double x) {
+  const uint64_t u = bits_of(x);
+  return ((uint32_t)(u >> 52) & 0x7ff) - 2u < 2045u ? of_bits(u - (1ull << 52)) : 0.5 * x;
+}
+I64_FN double quarter(double x) {
+  const uint64_t u = bits_of(x);
+  return ((uint32_t)(u >> 52) & 0x7ff) - 3u < 2044u ? of_bits(u - (2ull << 52)) : 0.25 * x;
+}
+// the integer part of a v in [1, 2^31), else 0
+I64_FN int trunc_pos(double v) {
+  const uint64_t u = bits_of(v);
+  const uint32_t e = (uint32_t)(u >> 52) - 1023u;
+  return e < 31u ? (int)(((u & 0xfffffffffffffull) | 0x10000000000000ull) >> (52 - e)) : 0;
+}
+I64_FN double from_float(float f) {
+  const uint32_t u = bits32(f), e = (u >> 23) & 255u;
+  if (e - 1u >= 254u) return (double)f;
+  return of_bits(((uint64_t)(u & 0x80000000u) << 32) | (((uint64_t)(u & 0x7fffffffu) << 29) + (896ull << 52)));
+}
 
 // ---------------------------------------------------------------- division
 I64_COLD double div_any(double a, double b) { return a / b; }
@@ -261,7 +282,7 @@ I64_FN double sqrt_(double a) {
   const uint64_t t0 = mul64x32(A, y) >> 31;
   const uint32_t s0 = (t0 >> 32) ? 0xffffffffu : (uint32_t)t0;  // Q1.31
   const int64_t d0 = (int64_t)(A - (uint64_t)s0 * s0);                             // a - s0^2, Q2.62
-  const uint64_t s1 = ((uint64_t)s0 << 31) + (uint64_t)(((int64_t)(int32_t)(d0 >> 13) * (int64_t)(uint64_t)y) >> 20);
+  const uint64_t s1 = ((uint64_t)s0 << 31) + (uint64_t)(((int64_t)(int32_t)(d0 >> 14) * (int64_t)(uint64_t)y) >> 19);
   const int64_t d1 = (int64_t)((A >> 2) - mulhi(s1, s1));                          // Q4.60
   const uint64_t s2 = s1 + (uint64_t)((d1 * (int64_t)(uint64_t)y) >> 31);          // Q2.62
   uint64_t s = s2 >> 9;                                                            // 54 bits
@@ -281,13 +302,8 @@ I64_FN double log_(double x) {
   const int k = (int)(h >> 20) - 1023;
   const uint32_t i = (h >> 13) & 127u;
   const uint64_t m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
-#ifdef __CUDA_ARCH__
-  const uint32_t ci = __ldg(&LOG_C[i]);
-  const uint64_t Ti = __ldg((const unsigned long long*)&LOG_T[i]);
-#else
-  const uint32_t ci = LOG_C_h[i];
-  const uint64_t Ti = LOG_T_h[i];
-#endif
+  const uint32_t ci = I64_AT(LOG_C, i);
+  const uint64_t Ti = I64_AT(LOG_T, i);
   const uint64_t z = (m * ci - 0x4000000000000000ull) << 2;  // exact, [0, 0.0087), Q0.64
   const uint32_t w = (uint32_t)(z >> 26);                      // 64 z, Q0.32
   // log1p(z) = z - z^2 (1/2 - z (1/3 - z/4 + z^2 (1/5 - z/6 + z^2/7 - z^3/8)))
@@ -335,11 +351,7 @@ I64_FN double exp_(double x) {
   const uint64_t y2 = mulhi(Y, Y);  // 2^14 y^2
   const uint64_t p = 0x8000000000000000ull + (mulhi(Y, 0x2aaaaaaaaaaaaaaaull) >> 7) + (mul64x32(y2, q) >> 14);
   const uint64_t e1 = (Y >> 7) + (mulhi(y2, p) >> 14);
-#ifdef __CUDA_ARCH__
-  const uint64_t T = __ldg((const unsigned long long*)&EXP_T[j]);
-#else
-  const uint64_t T = EXP_T_h[j];
-#endif
+  const uint64_t T = I64_AT(EXP_T, j);
   const uint64_t v = T + mulhi(T, e1);  // Q1.63, [1, 2)
   return of_bits(((uint64_t)(1022 + k) << 52) + (v >> 11) + ((v >> 10) & 1));
 }

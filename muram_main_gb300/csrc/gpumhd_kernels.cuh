@@ -155,12 +155,12 @@ enum { P_D, P_V1, P_V2, P_V3, P_EI, P_B1, P_B2, P_B3, P_P, P_EK, P_PM, NPRIM };
 // then the residual's kinetic and magnetic pressure terms (src/mhdres_SR.C:310-317).
 template <class R>
 __device__ __forceinline__ void prim_from_cons(R d, R m1, R m2, R m3, R e, R& v1, R& v2, R& v3, R& ei) {
-  R dn = (R)1.0 / d;
+  R dn = d_div((R)1.0, d);
   v1 = m1 * dn;
   v2 = m2 * dn;
   v3 = m3 * dn;
   R vv = v1 * v1 + v2 * v2 + v3 * v3;
-  ei = e - (R)0.5 * vv * d;
+  ei = e - d_half(vv) * d;
 }
 
 // The 9 stored values of a cell (state and pressure), as loaded from memory.
@@ -213,8 +213,8 @@ __device__ __forceinline__ void prim_of_raw(const Raw9<R>& r, R* out) {
   out[P_B2] = b2;
   out[P_B3] = b3;
   out[P_P] = r.v[8];
-  out[P_EK] = (R)0.5 * d * vv;
-  out[P_PM] = (R)0.5 * bb;
+  out[P_EK] = d_half(d) * vv;
+  out[P_PM] = d_half(bb);
 }
 
 // The 12 directional quantities whose 4th-order derivative the residual takes
@@ -234,19 +234,20 @@ __device__ __forceinline__ void flux12(const R* p, int s, R* f, int fs) {
   const R pr = p[P_P * s], ekin = p[P_EK * s], pmag = p[P_PM * s];
   const R vel = D1 == 0 ? v1 : (D1 == 1 ? v2 : v3);
   const R mag = D1 == 0 ? b1 : (D1 == 1 ? b2 : b3);
-  const R p1 = D1 == 0 ? (R)1.0 : (R)0.0, p2 = D1 == 1 ? (R)1.0 : (R)0.0, p3 = D1 == 2 ? (R)1.0 : (R)0.0;
   const R mflx = vel * d;
   f[0 * fs] = mflx;
-  f[1 * fs] = mflx * v1 + p1 * pr;
-  f[2 * fs] = mflx * v2 + p2 * pr;
-  f[3 * fs] = mflx * v3 + p3 * pr;
+  f[1 * fs] = mflx * v1;
+  f[2 * fs] = mflx * v2;
+  f[3 * fs] = mflx * v3;
+  f[(1 + D1) * fs] += pr;
   f[4 * fs] = vel * (ei + ekin + pr);
   const R F5 = vel * b1 - v1 * mag, F6 = vel * b2 - v2 * mag, F7 = vel * b3 - v3 * mag;
   f[5 * fs] = Dirs<D1>::fa == 5 ? F5 : F6;
   f[6 * fs] = Dirs<D1>::fb == 7 ? F7 : F6;
-  f[7 * fs] = mag * b1 - p1 * pmag;
-  f[8 * fs] = mag * b2 - p2 * pmag;
-  f[9 * fs] = mag * b3 - p3 * pmag;
+  f[7 * fs] = mag * b1;
+  f[8 * fs] = mag * b2;
+  f[9 * fs] = mag * b3;
+  f[(7 + D1) * fs] -= pmag;
   f[10 * fs] = Dirs<D1>::d2 == 0 ? b1 : b2;
   f[11 * fs] = Dirs<D1>::d3 == 1 ? b2 : b3;
 }
@@ -278,20 +279,9 @@ __device__ __forceinline__ void deriv12(float* Dq, const float* fm2, const float
 // 741-765): the direction's curl B parts accumulate in cb; the last direction
 // (z) adds the ohmic heating eta*|cb|^2 to Racc[4] before its residual; lap3
 // is eta times the fourth-order second derivative of B along the direction.
-template <class R, int D1, bool ETA = false>
+template <class R, int D1, bool ETA = false, bool FIRST = false>
 __device__ __forceinline__ void apply_direction(R* Racc, const R* Dq, const R* cen, R lf, R eta = (R)0,
                                                 R* cb = nullptr, const R* lap3 = nullptr) {
-  R res[NV];
-  res[0] = (R)0.0 - Dq[0];
-  res[1] = (R)0.0 - Dq[1];
-  res[2] = (R)0.0 - Dq[2];
-  res[3] = (R)0.0 - Dq[3];
-  res[4] = (R)0.0 - Dq[4];
-  res[5] = (R)0.0;
-  res[6] = (R)0.0;
-  res[7] = (R)0.0;
-  res[Dirs<D1>::fa] = (R)0.0 - Dq[5];
-  res[Dirs<D1>::fb] = (R)0.0 - Dq[6];
   const R dB2 = Dq[10], dB3 = Dq[11];
   const R Bd1 = cen[P_B1 + D1];
   const R Bd2 = cen[P_B1 + Dirs<D1>::d2], Bd3 = cen[P_B1 + Dirs<D1>::d3];
@@ -302,10 +292,16 @@ __device__ __forceinline__ void apply_direction(R* Racc, const R* Dq, const R* c
   const R lrt0 = lf * Dq[7] + ((R)1.0 - lf) * cbb[0];
   const R lrt1 = lf * Dq[8] + ((R)1.0 - lf) * cbb[1];
   const R lrt2 = lf * Dq[9] + ((R)1.0 - lf) * cbb[2];
-  res[1] += lrt0;
-  res[2] += lrt1;
-  res[3] += lrt2;
-  res[4] += cen[P_V1] * lrt0 + cen[P_V2] * lrt1 + cen[P_V3] * lrt2;
+  // Racc += (0 - D(F)) + Lorentz terms; FIRST: Racc is zero and not read
+  R res[NV];
+  res[0] = -Dq[0];
+  res[1] = lrt0 - Dq[1];
+  res[2] = lrt1 - Dq[2];
+  res[3] = lrt2 - Dq[3];
+  res[4] = (cen[P_V1] * lrt0 + cen[P_V2] * lrt1 + cen[P_V3] * lrt2) - Dq[4];
+  res[5 + D1] = (R)0.0;
+  res[Dirs<D1>::fa] = -Dq[5];
+  res[Dirs<D1>::fb] = -Dq[6];
   if (ETA) {
     const R signd1 = D1 == 1 ? (R)1.0 : (R)-1.0;
     cb[Dirs<D1>::d2] += signd1 * dB3;
@@ -316,7 +312,10 @@ __device__ __forceinline__ void apply_direction(R* Racc, const R* Dq, const R* c
     res[7] += lap3[2];
   }
 #pragma unroll
-  for (int q = 0; q < NV; q++) Racc[q] += res[q];
+  for (int q = 0; q < NV; q++) {
+    if (FIRST) Racc[q] = res[q];
+    else if (ETA || q != 5 + D1) Racc[q] += res[q];
+  }
 }
 
 // eta times the fourth-order second derivative of B along a direction of
@@ -333,14 +332,14 @@ __device__ __forceinline__ void eta_lap(const Consts& c, const R* __restrict__ U
   }
 }
 
-template <class R, int D1, bool ETA = false>
+template <class R, int D1, bool ETA = false, bool FIRST = false>
 __device__ __forceinline__ void add_direction(R* Racc, const R* __restrict__ fm2, const R* __restrict__ fm1,
                                               const R* __restrict__ fp1, const R* __restrict__ fp2, R w1,
                                               R w2, const R* cen, R lf, R eta = (R)0, R* cb = nullptr,
                                               const R* lap3 = nullptr) {
   R Dq[NF];
   deriv12(Dq, fm2, fm1, fp1, fp2, w1, w2);
-  apply_direction<R, D1, ETA>(Racc, Dq, cen, lf, eta, cb, lap3);
+  apply_direction<R, D1, ETA, FIRST>(Racc, Dq, cen, lf, eta, cb, lap3);
 }
 
 // ------------------------------------------------------------ stage kernel
@@ -411,11 +410,11 @@ __device__ __forceinline__ void rk_update(const Consts& c, Rem<R>* __restrict__ 
 // Boris factor of MHD_Residual's Lorentz-force blend at a cell (src/mhdres_SR.C:310-323).
 template <class R>
 __device__ __forceinline__ R boris_lf(const R* cen, R inv_va2max) {
-  const R dn = (R)1.0 / cen[P_D];
+  const R dn = d_div((R)1.0, cen[P_D]);
   const R bb = cen[P_B1] * cen[P_B1] + cen[P_B2] * cen[P_B2] + cen[P_B3] * cen[P_B3];
   const R va2 = bb * dn;
   const R x2 = va2 * inv_va2max, x4 = x2 * x2, s = (R)1.0 + x2;
-  return s / (s + x4);
+  return d_div(s, s + x4);
 }
 
 // Sources and semi-relativistic (Boris) correction added to the residual Racc
@@ -425,22 +424,25 @@ template <class R>
 __device__ __forceinline__ void stage_sources(R* Racc, const R* cen, R gx, R inv_va2max, R invRdt) {
   const R rh = cen[P_D], vx = cen[P_V1], vy = cen[P_V2], vz = cen[P_V3];
   const R bx = cen[P_B1], by = cen[P_B2], bz = cen[P_B3];
+  // the radiative term is zero times dn / max(dn, 0), dn the radiative limit
+  // over the internal energy: nothing for a positive finite dn, else NaN
   R dn = invRdt * cen[P_EI];
-  R efaci = (dn > (R)0 && dn < (R)INFINITY) ? (R)1.0 : dn / d_fmax(dn, (R)0.0);
-  dn = gx * rh - (R)0.0;
+  const bool rad_ok = d_lt((R)0, dn) && d_lt(dn, (R)INFINITY);
+  dn = gx * rh;
   const R edmp = dn * vx;
   Racc[1] += dn;
-  Racc[4] += edmp + (R)0.0 * efaci;
+  Racc[4] += edmp;
+  if (!rad_ok) Racc[4] = (R)NAN;
   const R rd = Racc[0];
   R fx = Racc[1], fy = Racc[2], fz = Racc[3];
   const R bb = bx * bx + by * by + bz * bz;
-  const R va2 = bb / rh;
+  const R va2 = d_div(bb, rh);
   const R x2 = va2 * inv_va2max, x4 = x2 * x2;
-  const R bf = x4 / ((R)1 + x2 + x4);
+  const R bf = d_div(x4, (R)1 + x2 + x4);
   fx -= vx * rd;
   fy -= vy * rd;
   fz -= vz * rd;
-  const R q = (fx * bx + fy * by + fz * bz) / d_fmax(tiny100<R>(), bb);
+  const R q = d_div(fx * bx + fy * by + fz * bz, d_fmax(tiny100<R>(), bb));
   const R b0 = -bf * (fx - q * bx), b1 = -bf * (fy - q * by), b2 = -bf * (fz - q * bz);
   const R b3 = b0 * vx + b1 * vy + b2 * vz;
   Racc[1] += b0;
@@ -603,13 +605,10 @@ __global__ void __launch_bounds__(TX* TY, 2) k_stage(Consts c, const R* __restri
     }
     __syncthreads();
     if (active) {
-      R Racc[NV];
+      R Racc[NV];  // fused stage: written by the first direction
       if (RESID) {
 #pragma unroll
         for (int q = 0; q < NV; q++) Racc[q] = base[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < NV; q++) Racc[q] = (R)0.0;
       }
       // Boris factor at the cell (src/mhdres_SR.C:310-323)
       const R lf = boris_lf<R>(cen, inv_va2max);
@@ -626,7 +625,7 @@ __global__ void __launch_bounds__(TX* TY, 2) k_stage(Consts c, const R* __restri
           load_cell(fb + CW, n2);
           load_cell(fb + 2 * CW, n3);
           if (ETA) eta_lap<R>(c, Uin, id, 1u, 0, cen, lap);
-          add_direction<R, 0, ETA>(Racc, n0, n1, n2, n3, w1x, w2x, cen, lf, kk_.eta, cb, lap);
+          add_direction<R, 0, ETA, !RESID>(Racc, n0, n1, n2, n3, w1x, w2x, cen, lf, kk_.eta, cb, lap);
         }
         {
           const R* fb = FY + ((ty + 2) * TX + tx) * CW;
@@ -664,7 +663,7 @@ __global__ void __launch_bounds__(TX* TY, 2) k_stage(Consts c, const R* __restri
         if (write_pres) {
           R v1, v2, v3, ei;
           prim_from_cons(un[0], un[1], un[2], un[3], un[4], v1, v2, v3, ei);
-          const R pr = eos_pres(c, un[0], ei, (R)1.0 / un[0]);
+          const R pr = eos_pres(c, un[0], ei, d_div((R)1.0, un[0]));
           store_scalar<R, true>(g, Pout, i, j, k, im, pr);
         }
       }
@@ -721,36 +720,56 @@ __device__ __forceinline__ void tvd_cell(const Consts& c, const Raw9<R>& r, R hb
   t.hb = hb;
   t.ht = ht;
   t.qt = qt;
-  R dn = (R)1.0 / d;
+  R dn = d_div((R)1.0, d);
   v1 = v1 * dn;
   v2 = v2 * dn;
   v3 = v3 * dn;
   R vv = v1 * v1 + v2 * v2 + v3 * v3;
   R bb = b5 * b5 + b6 * b6 + b7 * b7;
-  e = e * dn - (R)0.5 * vv;
+  e = e * dn - d_half(vv);
   t.vsqr = vv;
   t.bsqr = bb;
   vv = d_sqrt(vv);
   R va2 = bb * dn;
   R x2 = va2 * inv_va2max, x4 = x2 * x2, s = (R)1.0 + x2;
-  R lf = s / (s + x4);
+  R lf = d_div(s, s + x4);
   R cs2 = (R)(5.0 / 3.0) * r.v[8] * dn;
-  R cfast = d_sqrt(va2 + cs2);
   const R CZ = k.CZ;
-  R CME = ((R)1.0 - CZ) * ((R)(vv >= k.CME_thresh * cfast));
+  // FP64: with CZ = 1 (full optical depth) the Mach-number damping CME is zero
+  const bool mach = !std::is_same<R, double>::value || CZ != (R)1.0;
+  R CME = (R)0.0;
+  if (mach) {
+    R cfast = d_sqrt(va2 + cs2);
+    CME = ((R)1.0 - CZ) * ((R)(vv >= k.CME_thresh * cfast));
+  }
   dn = d * d;
-  R rf = smin(lf, dn / (dn + k.rho_lev));
+  R rf = smin(lf, d_div(dn, dn + k.rho_lev));
   R hh = (R)1.0 - t.hb - t.ht;
-  R cf = t.hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + ((R)1.0 - rf) * k.tvd_cs[2]) * hh + t.ht * k.tvd_cs[3];
+  const R h0 = k.tvd_h[0], h1 = k.tvd_h[1], h2 = k.tvd_h[2], h3 = k.tvd_h[3];
+  R cf;
+  // FP64: the boundary profiles are zero but for the cells next to the
+  // vertical boundaries; there their terms add nothing and hh is 1
+  if (std::is_same<R, double>::value && t.hb == (R)0.0 && t.ht == (R)0.0) {
+    const R ro = (R)1.0 - rf;
+    cf = rf * k.tvd_cs[1] + ro * k.tvd_cs[2];
+    const R a1 = rf * h1, a2 = ro * h2;
+    t.he = a1 + a2;
+    t.hv = a1 + a2 * k.pm_v;
+    t.hB = a1 + a2 * k.pm_B;
+  } else {
+    cf = t.hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + ((R)1.0 - rf) * k.tvd_cs[2]) * hh + t.ht * k.tvd_cs[3];
+    t.he = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2) * hh + t.ht * h3;
+    t.hv = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2 * k.pm_v) * hh + t.ht * h3 * k.pm_v;
+    t.hB = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2 * k.pm_B) * hh + t.ht * h3 * k.pm_B;
+  }
   cf = smax(cf, CME);
   cs2 *= cf * cf;
   t.cm = (R)0.0 + vv + d_sqrt(smax(cs2, lf * (cs2 + va2)));
-  const R h0 = k.tvd_h[0], h1 = k.tvd_h[1], h2 = k.tvd_h[2], h3 = k.tvd_h[3];
-  t.he = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2) * hh + t.ht * h3;
-  t.hv = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2 * k.pm_v) * hh + t.ht * h3 * k.pm_v;
-  t.hB = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2 * k.pm_B) * hh + t.ht * h3 * k.pm_B;
-  t.he *= ((R)1.0 - CME);
-  t.hv *= ((R)1.0 - CME);
+  if (mach) {
+    t.he *= ((R)1.0 - CME);
+    t.hv *= ((R)1.0 - CME);
+    t.hB *= ((R)1.0 - CME);
+  }
   t.BC2 = (R)1.0 - lf;
   t.hd = (R)0;
   if (hyper) {
@@ -784,7 +803,7 @@ __device__ __forceinline__ void tvd_slope(const Consts& c, const TCell<R>& a, co
   for (int v = 0; v < NV; v++) {
     R sl = b.q[v] - a.q[v];
     R sr = n.q[v] - b.q[v];
-    R slm = (R)0.25 * (sl + sr);
+    R slm = d_quarter(sl + sr);
     R lower = smin(smin(sl, sr), slm);
     R upper = smax(smax(sl, sr), slm);
     slp[v] = smax((R)0.0, lower) + smin((R)0.0, upper);
@@ -799,8 +818,8 @@ __device__ __forceinline__ void tvd_slope(const Consts& c, const TCell<R>& a, co
     slp[5] *= cf; slp[6] *= cf; slp[7] *= cf;
   }
   R qr = c.rho_log ? d_fabs(b.q[0] - n.q[0]) : d_fabs(d_log(b.q[0]) - d_log(n.q[0]));
-  if (qr > k.q_rho_max) slp[0] = (R)0.0;
-  if (k.has_vmax_lim && b.vsqr > vsqr_diff) { slp[1] = (R)0.0; slp[2] = (R)0.0; slp[3] = (R)0.0; }
+  if (d_lt(k.q_rho_max, qr)) slp[0] = (R)0.0;
+  if (k.has_vmax_lim && d_lt(vsqr_diff, b.vsqr)) { slp[1] = (R)0.0; slp[2] = (R)0.0; slp[3] = (R)0.0; }
 }
 
 // Interface flux between cells a (index ia) and b, plus its resistive-heating
@@ -815,7 +834,7 @@ __device__ __forceinline__ void tvd_flux(const Consts& c, const TCell<R>& am, co
     R sl = b.q[v] - a.q[v];
     R sl_lim = b.q[v] - a.q[v] - (sa[v] + sb[v]);
     R dn = (v >= 1 && v <= 3) ? a.hv : ((v >= 5) ? a.hB : a.he);
-    R rf = d_fabs(sl_lim) / smax(tiny100<R>(), d_fabs(sl));
+    R rf = d_div(d_fabs(sl_lim), smax(tiny100<R>(), d_fabs(sl)));
     R cf = smax((R)0.0, smin(sl_lim, sl)) + smin((R)0.0, smax(sl_lim, sl));
     F[v] = smax((R)0.0, (R)1.0 + dn * (rf - (R)1.0)) * cf;
   }
@@ -841,7 +860,7 @@ __device__ __forceinline__ void tvd_flux(const Consts& c, const TCell<R>& am, co
   R f0 = F[0], f1 = F[1], f2 = F[2], f3 = F[3], f4 = F[4];
   R u[5];
 #pragma unroll
-  for (int v = 0; v < 5; v++) u[v] = (R)0.5 * (a.q[v] + sa[v] + b.q[v] - sb[v]);
+  for (int v = 0; v < 5; v++) u[v] = d_half(a.q[v] + sa[v] + b.q[v] - sb[v]);
   if (c.rho_log) {
     u[0] = d_exp(u[0]);
     f0 *= u[0];
@@ -854,7 +873,8 @@ __device__ __forceinline__ void tvd_flux(const Consts& c, const TCell<R>& am, co
   f2 *= u[0]; f2 += u[2] * min_cz;
   f3 *= u[0]; f3 += u[3] * min_cz;
   f4 *= u[0];
-  f4 += (u[4] * min_cz) + a.qt * (u[1] * f1 + u[2] * f2 + u[3] * f3);
+  if (std::is_same<R, double>::value && a.qt == (R)1.0) f4 += (u[4] * min_cz) + (u[1] * f1 + u[2] * f2 + u[3] * f3);
+  else f4 += (u[4] * min_cz) + a.qt * (u[1] * f1 + u[2] * f2 + u[3] * f3);
   F[0] = f0; F[1] = f1; F[2] = f2; F[3] = f3; F[4] = f4;
   if (DIR == 0 && !c.g.periodic_x) {
     if (ia == sz - GH - 1) F[5] = (R)0.0;
@@ -887,10 +907,11 @@ __device__ __forceinline__ void tvd_update(const Consts& c, R dtt, const R* Fp, 
   R res[NV];
 #pragma unroll
   for (int v = 0; v < NV; v++) res[v] = dtt * (Fp[v] - Fm[v]);
-  res[4] += ((R)1.0 - c0.qt) * (res[1] * c0.q[1] + res[2] * c0.q[2] + res[3] * c0.q[3]);
+  if (!std::is_same<R, double>::value || c0.qt != (R)1.0)  // at qt = 1 it adds nothing
+    res[4] += ((R)1.0 - c0.qt) * (res[1] * c0.q[1] + res[2] * c0.q[2] + res[3] * c0.q[3]);
   if (DIAG) dg->d[7 * N + id] += res[4] * dg->idt_full;
   {
-    R dn = (res[1] * c0.q[5] + res[2] * c0.q[6] + res[3] * c0.q[7]) / smax(tiny100<R>(), c0.bsqr);
+    R dn = d_div(res[1] * c0.q[5] + res[2] * c0.q[6] + res[3] * c0.q[7], smax(tiny100<R>(), c0.bsqr));
     R b0 = -c0.BC2 * (res[1] - dn * c0.q[5]);
     R b1 = -c0.BC2 * (res[2] - dn * c0.q[6]);
     R b2 = -c0.BC2 * (res[3] - dn * c0.q[7]);
@@ -899,7 +920,7 @@ __device__ __forceinline__ void tvd_update(const Consts& c, R dtt, const R* Fp, 
     if (DIAG) dg->d[5 * N + id] += b3 * dg->idt_full;
   }
   {
-    R qres = (R)0.5 * (qp + qm) * c0.qt;
+    R qres = d_half(qp + qm) * c0.qt;
     res[4] += dtt * qres;
     if (DIAG) dg->d[8 * N + id] += dg->dt_fac * qres;
   }
@@ -929,7 +950,7 @@ __device__ __forceinline__ void tvd_update(const Consts& c, R dtt, const R* Fp, 
   for (int v = 0; v < NV; v++) u[v] = u_in[v] + res[v];
   u[0] = smax((R)kk_.rho_min, u[0]);
   const R eb = u[4];
-  u[4] = smax(u[4], kk_.eps_min * u[0] + (R)0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) / u[0]);
+  u[4] = smax(u[4], kk_.eps_min * u[0] + d_div(d_half(u[1] * u[1] + u[2] * u[2] + u[3] * u[3]), u[0]));
   if (DIAG) {
     dg->d[6 * N + id] += (u[4] - eb) * dg->idt_full;
     dg->d[9 * N + id] += dg->dt_fac * ((R)0.5 * (qvp + qvm) * c0.qt);
@@ -1037,7 +1058,7 @@ __global__ void __launch_bounds__(FIN_BX* FIN_BY, FinBlocks<R>::v) k_step_finish
         }
       R v1, v2, v3, ei;
       prim_from_cons(u[0], u[1], u[2], u[3], u[4], v1, v2, v3, ei);
-      const R pr = eos_pres(c, u[0], ei, (R)1.0 / u[0]);
+      const R pr = eos_pres(c, u[0], ei, d_div((R)1.0, u[0]));
       Pout[id] = pr;
       const Images im = images_of(g, i, j, k, true);
       if (im.xa >= 0 || im.ya >= 0 || im.za >= 0) {
@@ -1059,13 +1080,13 @@ __global__ void __launch_bounds__(FIN_BX* FIN_BY, FinBlocks<R>::v) k_step_finish
       R cmv = cmax_cell<R>(u[0], v1, v2, v3, u[5], u[6], u[7], pr, inv_va2max);
       acc.cmax = smax(acc.cmax, cmv);
       R vabs = d_sqrt(v1 * v1 + v2 * v2 + v3 * v3);
-      R cs = (R)(5 / 3.) * pr / u[0];
-      R ee = ei / u[0];
+      R cs = d_div((R)(5 / 3.) * pr, u[0]);
+      R ee = d_div(ei, u[0]);
       acc.v = d_fmax(acc.v, vabs);
       acc.cs = d_fmax(acc.cs, cs);
       acc.e = d_fmax(acc.e, ee);
-      if (vabs >= vlim95) acc.nv++;
-      if (ee >= elim95) acc.ne++;
+      if (!d_lt(vabs, vlim95) && vabs == vabs) acc.nv++;
+      if (!d_lt(ee, elim95) && ee == ee) acc.ne++;
     }
   }
   acc.flush(dyn);
@@ -1278,7 +1299,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_cons_to_prim(Consts c, 
     R d = U[id];
     R v1, v2, v3, ei;
     prim_from_cons(d, U[N + id], U[2 * N + id], U[3 * N + id], U[4 * N + id], v1, v2, v3, ei);
-    const R dn = (R)1.0 / d;
+    const R dn = d_div((R)1.0, d);
     R pr, tm, ne, ri, am;
     c2p_outputs(c, d, ei, dn, pr, tm, ne, ri, am);
     U[N + id] = v1;
@@ -1305,7 +1326,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_aux_of_snapshot(Consts 
   const unsigned N = c.g.N32;
   for (unsigned id = gs_first(); id < N; id += gs_step()) {
     const R d = T[id], ei = Ne[id];
-    const R dn = (R)1.0 / d;
+    const R dn = d_div((R)1.0, d);
     R pr, tm, ne, ri, am;
     c2p_outputs(c, d, ei, dn, pr, tm, ne, ri, am);
     T[id] = tm; Ne[id] = ne; Ri[id] = ri; Am[id] = am;
@@ -1326,20 +1347,20 @@ __global__ void k_init_pass(Consts c, const R* __restrict__ U, R* __restrict__ P
     R d = U[id];
     R v1, v2, v3, ei;
     prim_from_cons(d, U[N + id], U[2 * N + id], U[3 * N + id], U[4 * N + id], v1, v2, v3, ei);
-    R pr = eos_pres(c, d, ei, (R)1.0 / d);
+    R pr = eos_pres(c, d, ei, d_div((R)1.0, d));
     P[id] = pr;
     int i, j, k;
     node_ijk(g, id, i, j, k);
     if (i >= GH && i < GH + g.nx && j >= GH && j < GH + g.ny && k >= GH && k < GH + g.nz) {
       cm_loc = smax(cm_loc, cmax_cell<R>(d, v1, v2, v3, U[5 * N + id], U[6 * N + id], U[7 * N + id], pr, inv_va2max));
       R vabs = d_sqrt(v1 * v1 + v2 * v2 + v3 * v3);
-      R cs = (R)(5 / 3.) * pr / d;
-      R ee = ei / d;
+      R cs = d_div((R)(5 / 3.) * pr, d);
+      R ee = d_div(ei, d);
       sv = d_fmax(sv, vabs);
       sc = d_fmax(sc, cs);
       se = d_fmax(se, ee);
-      if (vabs >= vlim95) nv++;
-      if (ee >= elim95) ne++;
+      if (!d_lt(vabs, vlim95) && vabs == vabs) nv++;
+      if (!d_lt(ee, elim95) && ee == ee) ne++;
     }
   }
   R m = warp_max_nonnan(cm_loc);
@@ -1373,12 +1394,12 @@ __global__ void k_adjust_stats(Consts c, const R* __restrict__ U, const R* __res
     const unsigned id = cidx32(g, i, j, k);
     R d = U[id], v1 = U[N + id], v2 = U[2 * N + id], v3 = U[3 * N + id], ei = U[4 * N + id];
     R vabs = d_sqrt(v1 * v1 + v2 * v2 + v3 * v3);
-    R ee = ei / d;
+    R ee = d_div(ei, d);
     sv = d_fmax(sv, vabs);
-    sc = d_fmax(sc, (R)(5 / 3.) * P[id] / d);
+    sc = d_fmax(sc, d_div((R)(5 / 3.) * P[id], d));
     se = d_fmax(se, ee);
-    if (vabs >= vlim95) nv++;
-    if (ee >= elim95) ne++;
+    if (!d_lt(vabs, vlim95) && vabs == vabs) nv++;
+    if (!d_lt(ee, elim95) && ee == ee) ne++;
   }
   R a1 = warp_max_nonnan(sv), a2 = warp_max_nonnan(sc), a3 = warp_max_nonnan(se);
   for (int o = 16; o > 0; o >>= 1) {
@@ -1548,7 +1569,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_source_integrate(Consts
 #pragma unroll
     for (int v = 0; v < NV; v++) { r[v] = Res[(unsigned)v * N + id]; u[v] = U[(unsigned)v * N + id]; }
     R dn = invRdt * u[4];
-    R efaci = dn / d_fmax(dn, (R)0.0);
+    R efaci = d_div(dn, d_fmax(dn, (R)0.0));
     dn = kc<R>(c).gx * u[0] - (R)0.0;
     R edmp = dn * u[1];
     r[1] += dn;
@@ -1556,13 +1577,13 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_source_integrate(Consts
     const R rh = u[0], rd = r[0], vx = u[1], vy = u[2], vz = u[3], bx = u[5], by = u[6], bz = u[7];
     R fx = r[1], fy = r[2], fz = r[3];
     const R bb = bx * bx + by * by + bz * bz;
-    const R va2 = bb / rh;
+    const R va2 = d_div(bb, rh);
     const R x2 = va2 * inv_va2max, x4 = x2 * x2;
-    const R bf = x4 / ((R)1 + x2 + x4);
+    const R bf = d_div(x4, (R)1 + x2 + x4);
     fx -= vx * rd;
     fy -= vy * rd;
     fz -= vz * rd;
-    const R q = (fx * bx + fy * by + fz * bz) / d_fmax(tiny100<R>(), bb);
+    const R q = d_div(fx * bx + fy * by + fz * bz, d_fmax(tiny100<R>(), bb));
     const R b0 = -bf * (fx - q * bx), b1 = -bf * (fy - q * by), b2 = -bf * (fz - q * bz);
     const R b3 = b0 * vx + b1 * vy + b2 * vz;
     r[1] += b0; r[2] += b1; r[3] += b2; r[4] += b3;

@@ -420,13 +420,10 @@ __global__ void __launch_bounds__(TX* TY, 2)
     tm_deriv12(Dz, zcol(slot_add(s0, 3)), zcol(slot_add(s0, 4)), zcol(slot_add(s0, 1)), zcol(slot_add(s0, 2)),
                kk_.w1[2], kk_.w2[2]);
     if (active) {
-      R Racc[NV];
+      R Racc[NV];  // fused stage: written by the first direction
       if (RESID) {
 #pragma unroll
         for (int q = 0; q < NV; q++) Racc[q] = base[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < NV; q++) Racc[q] = (R)0.0;
       }
       // Boris factor at the cell (src/mhdres_SR.C:310-323)
       const R lf = boris_lf<R>(cen, inv_va2max);
@@ -440,7 +437,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
           const R* fb = FX + (ty * L::BX + tx + 2) * CW;
           deriv12(Dq, fb - 2 * CW, fb - CW, fb + CW, fb + 2 * CW, kk_.w1[0], kk_.w2[0]);
           if (ETA) eta_lap<R>(c, Ug, id, 1u, 0, cen, lap);
-          apply_direction<R, 0, ETA>(Racc, Dq, cen, lf, kk_.eta, cb, lap);
+          apply_direction<R, 0, ETA, !RESID>(Racc, Dq, cen, lf, kk_.eta, cb, lap);
         }
         {
           R Dq[NF];
@@ -471,7 +468,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
         if (write_pres) {
           R v1, v2, v3, ei;
           prim_from_cons(un[0], un[1], un[2], un[3], un[4], v1, v2, v3, ei);
-          eos_pres_begin(c, un[0], ei, (R)1.0 / un[0], plook);
+          eos_pres_begin(c, un[0], ei, d_div((R)1.0, un[0]), plook);
           pend = true;
         }
       }

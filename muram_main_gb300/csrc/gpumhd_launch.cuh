@@ -109,16 +109,16 @@ inline int grid_for(long long n, int block) {
 
 // z planes per stage block (bxy column tiles, nz planes, res resident blocks).
 // A block's time is about its planes plus two (FP64 one) for its prologue (four
-// z-flux planes) per wave of resident blocks; where two blocks share an SM
-// (FP32), a first wave of at most one block per SM takes 0.85 of a full wave's
-// time per plane, and over many waves the last, partly filled one is half
-// hidden.  Small boxes therefore march short chunks, down
-// to one plane (16 x 12 x 8 FP32: 19.2 us per stage with 4 planes, 11.2 with
-// 1; 96^3 FP32: 66 us with 24 planes, 48 with 12), large ones the longest chunks that fill the last wave.  A
-// shorter chunk has to be 1 % better to be taken.
+// z-flux planes) per wave of resident blocks; a first wave of at most one block
+// per SM takes 0.85 (FP64 0.7) of a full wave's time per plane, and over many
+// waves the last, partly filled one is half hidden.  Small boxes therefore
+// march short chunks, down to one plane (FP32 16 x 12 x 8: 19.2 us per stage
+// with 4 planes, 11.2 with 1; 96^3: 66 us with 24, 48 with 12; FP64 64^3: 0.39
+// ms with 16, 0.33 with 8), large ones the longest chunks that fill the last
+// wave.  A shorter chunk has to be 1 % better to be taken.
 template <class R>
 inline int stage_chunk(long long bxy, int nz, int res) {
-  const double half = sizeof(R) == 4 ? 0.85 : 1.0, first = sizeof(R) == 4 ? 2.0 : 1.0;
+  const double half = sizeof(R) == 4 ? 0.85 : 0.7, first = sizeof(R) == 4 ? 2.0 : 1.0;
   int best_zc = nz;
   double best = 1e300;
   for (int nzc = 1; nzc <= nz && nzc <= 1024; nzc++) {
@@ -140,7 +140,7 @@ inline int stage_chunk(long long bxy, int nz, int res) {
 // second wave start in pairs on the SMs that come free.  Measured, y sweep:
 // FP32 16 x 12 x 8 19.4 us with 32 cells, 11.1 with 2; 64^3 34.6 us with 32,
 // 19.0 with 4; 128^3 77 us with 32, 75 with 16; 192 x 128 x 256 179 us with
-// 32, 182 with 16, 198 with 64; FP64 64^3 0.99 ms with 32, 0.51 with 8.
+// 32, 182 with 16, 198 with 64; FP64 64^3 0.63 ms with 32, 0.25 with 8.
 template <class R>
 inline int tvd_chunk(long long pencils, int n1, int most) {
   constexpr bool f32 = sizeof(R) == 4;
@@ -152,7 +152,7 @@ inline int tvd_chunk(long long pencils, int n1, int most) {
     const double w = (double)blocks / (152.0 * per_sm), full = floor(w);
     double waves;
     if (f32) waves = 1.75 * full + (w > full ? 0.7 + 1.05 * (w - full) : 0.0);
-    else waves = w <= 0.5 ? 0.5 : ceil(w);
+    else waves = w <= 0.5 ? 0.75 : ceil(w);
     const double cost = ((td < n1 ? td : n1) + (f32 ? 4.0 : 1.5)) * waves;
     if (cost < 0.99 * best) { best = cost; best_td = td; }
   }
@@ -160,6 +160,28 @@ inline int tvd_chunk(long long pencils, int n1, int most) {
 }
 
 #ifdef GPUMHD_LAUNCH_IMPL
+// Resident blocks per SM of a kernel that allocates tensor memory, from its
+// registers, shared memory and the 512 tensor-memory columns of an SM.  (The
+// occupancy query answers 1 for every such kernel, whatever its resources; two
+// blocks do run.)
+template <class K>
+inline cudaError_t tm_blocks_per_sm(int* out, K kernel, int threads, int smem, int tmem_cols) {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sm_smem = 0, sm_regs = 0, reserved = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&sm_regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  const int by_regs = sm_regs / (((a.numRegs + 7) / 8 * 8) * threads);
+  const int by_smem = sm_smem / (smem + (int)a.sharedSizeBytes + reserved);
+  int n = by_regs < by_smem ? by_regs : by_smem;
+  n = n < 512 / tmem_cols ? n : 512 / tmem_cols;
+  *out = n > 1 ? n : 1;
+  return cudaSuccess;
+}
+
 template <class R>
 int Launch<R>::stage_smem_bytes() {
   return (int)StageSmem<StageTile<R>::TX, StageTile<R>::TY>::template bytes<R>();
@@ -190,7 +212,7 @@ cudaError_t Launch<R>::setup() {
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_stage_tm<R, MX, MY, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_tm<R, MX, MY, false, false>, MX * MY, tb);
+  e = tm_blocks_per_sm(&per_sm, k_stage_tm<R, MX, MY, false, false>, MX * MY, tb, StageTm<R, MX, MY, false>::TMEM_COLS);
   if (e != cudaSuccess) return e;
   int per_sm_db = per_sm;
   if constexpr (sizeof(R) == 4) {
@@ -199,7 +221,7 @@ cudaError_t Launch<R>::setup() {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_stage_tm<R, MX, MY, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tdb);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_db, k_stage_tm<R, MX, MY, false, true>, MX * MY, tdb);
+    e = tm_blocks_per_sm(&per_sm_db, k_stage_tm<R, MX, MY, false, true>, MX * MY, tdb, StageTm<R, MX, MY, true>::TMEM_COLS);
     if (e != cudaSuccess) return e;
   }
   // the z chunking assumes the smaller residency of the two layouts

@@ -4,6 +4,7 @@
 #include <math.h>
 
 #include "gpumhd_stage_tm.cuh"
+#include "gpumhd_tvd_f32.cuh"
 #include "gpumhd_divb.cuh"
 #include "gpumhd_bnd.cuh"
 #include "gpumhd_spitzer.cuh"
@@ -315,16 +316,26 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
     else k_tvd_sweep<R, 2, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr);
     return;
   }
-  const TvdDiag<R> nod{nullptr, (R)0, (R)0};
-  if (dir == 0 && mode == 0) {
-    // contiguous pencils: one cell per lane, 28 updates per warp
-    const long long warps = (long long)g.sy * g.sz * ((g.nx + 27) / 28);
-    long long nb = (warps * 32 + block - 1) / block;
-    if (nb > 152LL * 16) nb = 152LL * 16;   // grid-stride: a few waves of resident blocks
-    (Cc ? k_tvd_sweep_xlanes<R, true> : k_tvd_sweep_xlanes<R, false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Cc);
-    return;
+  // contiguous x pencils: one cell per lane, 28 updates per warp, grid-stride
+  // over a few waves of resident blocks
+  const long long warps = (long long)g.sy * g.sz * ((g.nx + 27) / 28);
+  long long nb = (warps * 32 + block - 1) / block;
+  if (nb > 152LL * 16) nb = 152LL * 16;
+  if constexpr (sizeof(R) == 4) {
+    if (c.rho_log) {
+      // at least one warp per segment (28 cells)
+      const long long least = ((g.nx + 27) / 28 + 3) / 4;
+      if (nb < least) nb = least;
+      if (dir == 0) (Cc ? k_tvd_xlanes_f32<true> : k_tvd_xlanes_f32<false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Cc);
+      else if (dir == 1) (Cc ? k_tvd_pencil_f32<1, true> : k_tvd_pencil_f32<1, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Cc);
+      else (Cc ? k_tvd_pencil_f32<2, true> : k_tvd_pencil_f32<2, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Cc);
+      return;
+    }
   }
-  if (dir == 0) (Cc ? k_tvd_sweep<R, 0, false, true> : k_tvd_sweep<R, 0, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
+  const TvdDiag<R> nod{nullptr, (R)0, (R)0};
+  if (dir == 0) {
+    (Cc ? k_tvd_sweep_xlanes<R, true> : k_tvd_sweep_xlanes<R, false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Cc);
+  }
   else if (dir == 1) (Cc ? k_tvd_sweep<R, 1, false, true> : k_tvd_sweep<R, 1, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
   else (Cc ? k_tvd_sweep<R, 2, false, true> : k_tvd_sweep<R, 2, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
 }

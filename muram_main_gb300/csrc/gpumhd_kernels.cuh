@@ -114,6 +114,13 @@ __device__ __forceinline__ void for_col_images(unsigned id, const ColImg& ci, in
     }
   }
 }
+// Element at a 32-bit byte offset from a base pointer that is the same for the
+// whole grid (an array of a box is below 2^32 bytes): one offset register
+// serves the accesses to all eight arrays.
+template <class T>
+__device__ __forceinline__ T* at(T* base, unsigned off) {
+  return reinterpret_cast<T*>(reinterpret_cast<char*>(const_cast<typename std::remove_const<T>::type*>(base)) + off);
+}
 template <class R>
 __device__ __forceinline__ void store_state_col(const Geom& g, R* __restrict__ U, unsigned id, const ColImg& ci, int oz,
                                                 const R v[NV]) {
@@ -122,7 +129,7 @@ __device__ __forceinline__ void store_state_col(const Geom& g, R* __restrict__ U
     for (int q = 0; q < NV; q++) {
       R x = v[q];
       if (f && (q == 1 || q == 6 || q == 7)) x = -x;
-      U[t + (unsigned)q * g.N32] = x;
+      *at(U + q * g.N, t * (unsigned)sizeof(R)) = x;
     }
   });
 }

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
   auto finish_pressure = [&](int kp) {
     const R pr = eos_pres_end(plook);
     for_col_images(own0 + (unsigned)kp * plane, col_images(g, i, j, true), z_image_off(g, kp),
-                   [&](unsigned t, bool) { Pout[t] = pr; });
+                   [&](unsigned t, bool) { *at(Pout, t * (unsigned)sizeof(R)) = pr; });
     pend = false;
   };
   int s0 = 2;  // ring slot of plane k
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
       // RESID: U0 is the residual to add to (null: start from zero)
       if (!RESID || U0) {
 #pragma unroll
-        for (int q = 0; q < NV; q++) base[q] = U0[id + (unsigned)q * g.N32];
+        for (int q = 0; q < NV; q++) base[q] = *at(U0 + q * g.N, id * (unsigned)sizeof(R));
       } else {
 #pragma unroll
         for (int q = 0; q < NV; q++) base[q] = (R)0;
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
       if (c.has_spitzer) Racc[4] += ((const R*)c.spt_rsp)[id];
       if (RESID) {
 #pragma unroll
-        for (int q = 0; q < NV; q++) Res[id + (unsigned)q * g.N32] = Racc[q];
+        for (int q = 0; q < NV; q++) *at(Res + q * g.N, id * (unsigned)sizeof(R)) = Racc[q];
         const R cm = cmax_cell<R>(cen[P_D], cen[P_V1], cen[P_V2], cen[P_V3], cen[P_B1], cen[P_B2], cen[P_B3],
                                   cen[P_P], inv_va2max);
         if (cm > cm_acc) cm_acc = cm;  // a NaN speed is skipped, as the atomic maximum skips it

@@ -56,29 +56,15 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // One instruction each, within 1 ulp (rcp) and 2 ulp (2^x, x near 0), or 2^-23
 // relative (sqrt); subnormal arguments count as zero, which here are densities
 // and squares far below anything the floors let pass.
-__device__ __forceinline__ float rcp(float a) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ float sqrt_(float a) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
+__device__ __forceinline__ float rcp(float a) { return f_rcp(a); }
+__device__ __forceinline__ float sqrt_(float a) { return f_sqrt(a); }
 __device__ __forceinline__ float exp2_(float a) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
 
-// The eight state arrays and the pressure by their own base pointers, the same
-// for the whole grid, and a 32-bit byte offset per thread (a box has less than
-// 2^29 nodes): one address register instead of index arithmetic per access.
-template <class T>
-__device__ __forceinline__ T* at(T* base, unsigned off) {
-  return reinterpret_cast<T*>(reinterpret_cast<char*>(const_cast<typename std::remove_const<T>::type*>(base)) + off);
-}
+// The eight state arrays and the pressure at a byte offset (see at()).
 __device__ __forceinline__ void load9(const float* __restrict__ U, const float* __restrict__ P, long long N, unsigned off,
                                       Raw9<float>& r) {
 #pragma unroll

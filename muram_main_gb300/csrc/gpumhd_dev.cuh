@@ -488,7 +488,7 @@ __device__ __forceinline__ float eos_pres(const Consts& c, float d, float ei, fl
   i_e = max(0, min(c.N_eps - 2, i_e));
   const float fe = log1p_small(eps * __ldg(c.inv_exp_xeps + i_e) - 1.0f);
   const float fr = log1p_small(d * __ldg(c.inv_exp_xlr + i_d) - 1.0f);
-  const float4 q = __ldg(c.pquad + (long long)i_e * c.N_lr + i_d);
+  const float4 q = __ldg(c.pquad + ((unsigned)i_e * (unsigned)c.N_lr + (unsigned)i_d));
   return q.x * exp_small(fe * q.y + fr * q.z + fe * fr * q.w);
 }
 
@@ -579,7 +579,7 @@ __device__ __forceinline__ void eos_pres_begin(const Consts& c, float d, float e
   i_e = max(0, min(c.N_eps - 2, i_e));
   L.ix = __ldg(c.inv_exp_xeps + i_e);
   L.id = __ldg(c.inv_exp_xlr + i_d);
-  L.q = __ldg(c.pquad + (long long)i_e * c.N_lr + i_d);
+  L.q = __ldg(c.pquad + ((unsigned)i_e * (unsigned)c.N_lr + (unsigned)i_d));
   L.eps = eps;
   L.d = d;
   L.ready = 0;

@@ -100,6 +100,7 @@ __device__ __forceinline__ int z_image_off(const Geom& g, int k) {
 template <class F>
 __device__ __forceinline__ void for_col_images(unsigned id, const ColImg& ci, int oz, F f) {
   f(id, false);
+  if ((ci.ox | ci.oy | oz) == 0) return;  // most cells
   if (ci.ox) f(id + (unsigned)ci.ox, ci.xf != 0);
   if (ci.oy) {
     f(id + (unsigned)ci.oy, false);

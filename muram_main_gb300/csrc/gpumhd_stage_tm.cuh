@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
 
   // plane tiles: plane p is tile t = p - (zb - 2), slot t % NSLOT, phase (t / NSLOT) % 2
   const int p_first = zb - 2;
-  auto tile = [&](int p) { return reinterpret_cast<const R*>(sm + (size_t)((p - p_first) % L::NSLOT) * L::TILE); };
+  auto tile_at = [&](int sl) { return reinterpret_cast<const R*>(sm + (size_t)sl * L::TILE); };
   // test hook: the last plane's copy is never issued, so its wait runs out
   const int withheld = c.tm_withhold_last ? ze + 1 : -1;
   const long long wait_limit = c.tm_wait_cycles > 0 ? c.tm_wait_cycles : tm::WAIT_CYCLES;
@@ -310,10 +310,10 @@ __global__ void __launch_bounds__(TX* TY, 2)
     tm::tma_load_3d(dst + L::UB, &mapP, bx0, by0, p, &bar[sl]);
   };
   bool timed_out = false;
-  auto wait_tile = [&](int p) {
-    const int t = p - p_first;
-    if (!tm::mbar_wait(&bar[t % L::NSLOT], (unsigned)((t / L::NSLOT) & 1), wait_limit)) timed_out = true;
+  auto wait_slot = [&](int sl, unsigned phase) {
+    if (!tm::mbar_wait(&bar[sl], phase, wait_limit)) timed_out = true;
   };
+  auto slot_next = [](int sl) { return sl + 1 == L::NSLOT ? 0 : sl + 1; };
   // cell offsets inside a tile: own cell and halo cell
   const int o_own = (ty + 2) * L::BX + (tx + 2);
   const int o_halo = (hly + 2) * L::BX + (hlx + 2);
@@ -327,16 +327,25 @@ __global__ void __launch_bounds__(TX* TY, 2)
 
   if (tid == 0)
     for (int p = zb - 2; p < zb - 2 + L::NSLOT; p++) issue(p);
-  for (int p = zb - 2; p < zb + 2; p++) {
+  // slot and phase of the plane waited for next, counted along (not divided out
+  // of the plane's number): with the images' offsets formed once per column and
+  // skipped in one test, stages 1 / 2 708 / 725 -> 672 / 678 us at 128 x 384 x 384
+  int sl_n = 0;
+  unsigned ph_n = 0;
+  auto advance = [&]() {
+    sl_n = slot_next(sl_n);
+    if (sl_n == 0) ph_n ^= 1u;
+  };
+  for (int p = zb - 2; p < zb + 2; p++, advance()) {
     if (L::DB && p == zb + 1) {  // the fourth prologue plane takes the first plane's slot
       tm::tmem_wait_st();
       __syncthreads();
       if (tid == 0) issue(p);
     }
-    wait_tile(p);
+    wait_slot(sl_n, ph_n);
     __syncwarp();
     Raw9<R> r;
-    raw_at(tile(p), o_own, r);
+    raw_at(tile_at(sl_n), o_own, r);
     prim_of_raw<R, RESID>(r, prim);
     flux12<R, 2>(prim, 1, fl, 1);
     tm_store12(zcol(p - zb + 2), fl);
@@ -347,27 +356,29 @@ __global__ void __launch_bounds__(TX* TY, 2)
 
   const unsigned plane = (unsigned)g.sx * (unsigned)g.sy;
   const unsigned own0 = cidx32(g, i, j, 0);
+  const ColImg img = col_images(g, i, j, true);  // ghost images of the column's cells
   // The new state's pressure of plane k is looked up at the end of plane k
   // and stored during plane k+1, so the table loads overlap that plane's work.
   PresLookup<R> plook;
   bool pend = false;
   auto finish_pressure = [&](int kp) {
     const R pr = eos_pres_end(plook);
-    for_col_images(own0 + (unsigned)kp * plane, col_images(g, i, j, true), z_image_off(g, kp),
+    for_col_images(own0 + (unsigned)kp * plane, img, z_image_off(g, kp),
                    [&](unsigned t, bool) { *at(Pout, t * (unsigned)sizeof(R)) = pr; });
     pend = false;
   };
-  int s0 = 2;  // ring slot of plane k
-  for (int k = zb; k < ze; k++, s0 = slot_add(s0, 1)) {
+  int s0 = 2;           // z-flux ring slot of plane k
+  int sl_k = 2 % L::NSLOT;  // tile slot of plane k
+  for (int k = zb; k < ze; k++, s0 = slot_add(s0, 1), sl_k = slot_next(sl_k), advance()) {
     if (!L::DB && tid == 0 && k + 1 < ze) issue(k + 3);
     R* const FX = fx_of(L::DB ? ((k - zb) & 1) : 0);
     R* const FY = FX + 12 * L::FXN;
     // z flux of plane k+2 (all lanes: tensor-memory stores are warp-wide)
-    wait_tile(k + 2);
+    wait_slot(sl_n, ph_n);
     __syncwarp();
     {
       Raw9<R> r;
-      raw_at(tile(k + 2), o_own, r);
+      raw_at(tile_at(sl_n), o_own, r);
       prim_of_raw<R, RESID>(r, prim);
       flux12<R, 2>(prim, 1, fl, 1);
       tm_store12(zcol(slot_add(s0, 2)), fl);
@@ -375,7 +386,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
     // own cell: primitives and x / y fluxes; halo cell: its x or y flux
     R cen[NF];
     {
-      const R* T = tile(k);
+      const R* T = tile_at(sl_k);
       Raw9<R> r;
       raw_at(T, o_own, r);
       prim_of_raw<R, RESID>(r, cen);
@@ -464,7 +475,7 @@ __global__ void __launch_bounds__(TX* TY, 2)
         stage_sources<R>(Racc, cen, kk_.gx, inv_va2max, invRdt);
         R un[NV];
         rk_update<R>(c, Cc, id, stage, wdt, base, Racc, vmax, emax, un);
-        store_state_col<R>(g, Uout, id, col_images(g, i, j, true), z_image_off(g, k), un);
+        store_state_col<R>(g, Uout, id, img, z_image_off(g, k), un);
         if (write_pres) {
           R v1, v2, v3, ei;
           prim_from_cons(un[0], un[1], un[2], un[3], un[4], v1, v2, v3, ei);

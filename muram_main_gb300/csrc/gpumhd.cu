@@ -823,6 +823,22 @@ static int ensure_staging(gpumhd_ctx* ctx) {
   return GPUMHD_OK;
 }
 
+// A kernel's address of pinned host memory [p, p + bytes), or null: pageable
+// memory, or a range that is not one pinned piece (those go through a staging
+// buffer).
+static void* pinned_on_device(const void* p, size_t bytes) {
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, (const char*)p + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
+      (char*)b.devicePointer != (char*)a.devicePointer + (bytes - 1))
+    return nullptr;
+  return a.devicePointer;
+}
+
 // Host element type H: double (MURaM's default build) or float (SINGLE_PRECISION).
 template <class H>
 static int upload_impl(gpumhd_ctx* ctx, int which, const H* host) {
@@ -831,13 +847,18 @@ static int upload_impl(gpumhd_ctx* ctx, int which, const H* host) {
   int nf, rc;
   void* dst = field_ptr(ctx, which, &nf, &rc);
   if (rc) return fail(ctx, rc, "upload: bad field %d", which);
-  rc = ensure_staging(ctx);
-  if (rc) return rc;
   const long long N = ctx->c.g.N;
-  H* const stg = reinterpret_cast<H*>(ctx->staging);
-  CK(cudaMemcpyAsync(stg, host, sizeof(H) * nf * N, cudaMemcpyHostToDevice, ctx->stream));
-  if (ctx->f32) Launch<float>::aos_to_soa(N, nf, stg, (float*)dst, ctx->stream);
-  else Launch<double>::aos_to_soa(N, nf, stg, (double*)dst, ctx->stream);
+  const Geom& g = ctx->c.g;
+  const H* src = (const H*)pinned_on_device(host, sizeof(H) * nf * N);
+  const bool direct = src != nullptr;
+  if (!direct) {
+    rc = ensure_staging(ctx);
+    if (rc) return rc;
+    src = reinterpret_cast<const H*>(ctx->staging);
+    CK(cudaMemcpyAsync(ctx->staging, host, sizeof(H) * nf * N, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  if (ctx->f32) Launch<float>::aos_to_soa(g, nf, src, (float*)dst, direct, ctx->stream);
+  else Launch<double>::aos_to_soa(g, nf, src, (double*)dst, direct, ctx->stream);
   if (which == 0) {
     ctx->fused_ready = false;
     if (ctx->comp) CK(cudaMemsetAsync(ctx->comp, 0, sizeof(Rem<float>) * 8 * N, ctx->stream));
@@ -905,8 +926,8 @@ static int upload_async_impl(gpumhd_ctx* ctx, int which, const H* host) {
   CK(cudaMemcpyAsync(stg, host, sizeof(H) * nf * N, cudaMemcpyHostToDevice, ctx->s_in));
   CK(cudaEventRecord(ctx->ev_in_ready[b], ctx->s_in));
   CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_in_ready[b], 0));
-  if (ctx->f32) Launch<float>::aos_to_soa(N, nf, stg, (float*)dst, ctx->stream);
-  else Launch<double>::aos_to_soa(N, nf, stg, (double*)dst, ctx->stream);
+  if (ctx->f32) Launch<float>::aos_to_soa(ctx->c.g, nf, stg, (float*)dst, false, ctx->stream);
+  else Launch<double>::aos_to_soa(ctx->c.g, nf, stg, (double*)dst, false, ctx->stream);
   CK(cudaEventRecord(ctx->ev_in_free[b], ctx->stream));
   if (which == 0) {
     ctx->fused_ready = false;
@@ -938,8 +959,8 @@ static int download_async_impl(gpumhd_ctx* ctx, int which, H* host) {
   const int b = (int)(ctx->n_down++ & 1u);
   CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_out_free[b], 0));
   H* const stg = reinterpret_cast<H*>(ctx->astage_out[b]);
-  if (ctx->f32) Launch<float>::soa_to_aos(N, nf, (const float*)src, stg, ctx->stream);
-  else Launch<double>::soa_to_aos(N, nf, (const double*)src, stg, ctx->stream);
+  if (ctx->f32) Launch<float>::soa_to_aos(ctx->c.g, nf, (const float*)src, stg, false, ctx->stream);
+  else Launch<double>::soa_to_aos(ctx->c.g, nf, (const double*)src, stg, false, ctx->stream);
   rc = check_launch(ctx, 1);
   if (rc) return rc;
   CK(cudaEventRecord(ctx->ev_out_ready[b], ctx->stream));
@@ -962,15 +983,19 @@ static int download_impl(gpumhd_ctx* ctx, int which, H* host) {
   int nf, rc;
   void* src = field_ptr(ctx, which, &nf, &rc);
   if (rc) return fail(ctx, rc, "download: bad field %d", which);
-  rc = ensure_staging(ctx);
-  if (rc) return rc;
   const long long N = ctx->c.g.N;
-  H* const stg = reinterpret_cast<H*>(ctx->staging);
-  if (ctx->f32) Launch<float>::soa_to_aos(N, nf, (const float*)src, stg, ctx->stream);
-  else Launch<double>::soa_to_aos(N, nf, (const double*)src, stg, ctx->stream);
+  H* dst = (H*)pinned_on_device(host, sizeof(H) * nf * N);
+  const bool direct = dst != nullptr;
+  if (!direct) {
+    rc = ensure_staging(ctx);
+    if (rc) return rc;
+    dst = reinterpret_cast<H*>(ctx->staging);
+  }
+  if (ctx->f32) Launch<float>::soa_to_aos(ctx->c.g, nf, (const float*)src, dst, direct, ctx->stream);
+  else Launch<double>::soa_to_aos(ctx->c.g, nf, (const double*)src, dst, direct, ctx->stream);
   rc = check_launch(ctx, 1);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(host, stg, sizeof(H) * nf * N, cudaMemcpyDeviceToHost, ctx->stream));
+  if (!direct) CK(cudaMemcpyAsync(host, dst, sizeof(H) * nf * N, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return GPUMHD_OK;
 }

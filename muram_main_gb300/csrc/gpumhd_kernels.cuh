@@ -1712,16 +1712,63 @@ __global__ void k_fill_ghosts(Geom g, R* __restrict__ U, int nfield, int with_bc
   }
 }
 
-// Host cState (AoS, double) <-> device SoA (R)
-template <class R, class H>
-__global__ void k_aos_to_soa(long long N, int nf, const H* __restrict__ A, R* __restrict__ S) {
-  for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < N; id += (long long)gridDim.x * blockDim.x)
-    for (int v = 0; v < nf; v++) S[(long long)v * N + id] = (R)A[id * nf + v];
+// Host layout (records of nf values per node: cState's eight, or single fields;
+// H: double, or float as in a SINGLE_PRECISION build) <-> device arrays (R).
+// A may be device memory (a staging buffer) or pinned host memory, which the
+// kernel then reads or writes over the link itself: the conversion costs no pass
+// of its own (0.64 GB: 3.02 ms up and 3.30 down, as the copies alone take, against
+// 0.2 to 0.3 ms more through a staging buffer).  The link is busy with 38 blocks.
+// VEC: A is 16-byte aligned and nf is 8, so records move in 16-byte pieces;
+// downwards the lanes of a warp exchange values so that each of its stores
+// covers 512 contiguous bytes (one record per thread instead: 8 ms).
+template <class R, class H, bool VEC>
+__global__ void k_aos_to_soa(Geom g, int nf, const H* __restrict__ A, R* __restrict__ S) {
+  const unsigned N = g.N32;
+  for (unsigned id = gs_first(); id < N; id += gs_step()) {
+    if constexpr (VEC) {
+      constexpr int PR = 8 * sizeof(H) / 16, EP = 16 / sizeof(H);  // 16-byte pieces per record, values per piece
+      uint4 raw[PR];
+      const uint4* p = reinterpret_cast<const uint4*>(A) + (unsigned long long)id * PR;
+#pragma unroll
+      for (int q = 0; q < PR; q++) raw[q] = p[q];
+      const H* v = reinterpret_cast<const H*>(raw);
+#pragma unroll
+      for (int q = 0; q < PR * EP; q++) S[(unsigned)q * N + id] = (R)v[q];
+    } else {
+      for (int v = 0; v < nf; v++) S[(unsigned)v * N + id] = (R)A[(unsigned long long)id * nf + v];
+    }
+  }
 }
-template <class R, class H>
-__global__ void k_soa_to_aos(long long N, int nf, const R* __restrict__ S, H* __restrict__ A) {
-  for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < N; id += (long long)gridDim.x * blockDim.x)
-    for (int v = 0; v < nf; v++) A[id * nf + v] = (H)S[(long long)v * N + id];
+template <class R, class H, bool VEC>
+__global__ void k_soa_to_aos(Geom g, int nf, const R* __restrict__ S, H* __restrict__ A) {
+  const unsigned N = g.N32;
+  if constexpr (VEC) {
+    constexpr int PR = 8 * sizeof(H) / 16, EP = 16 / sizeof(H), RW = 32 / PR;  // records per warp store
+    const unsigned lane = threadIdx.x & 31u;
+    for (unsigned base = gs_first() - lane; base < N; base += gs_step()) {
+      const unsigned id = min(base + lane, N - 1u);
+      H v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = (H)S[(unsigned)q * N + id];
+#pragma unroll
+      for (int r = 0; r < PR; r++) {
+        const unsigned src = r * RW + lane / PR, piece = lane % PR;
+        uint4 raw;
+        H* w = reinterpret_cast<H*>(&raw);
+#pragma unroll
+        for (int e = 0; e < EP; e++)
+#pragma unroll
+          for (int q = 0; q < PR; q++) {
+            const H x = __shfl_sync(0xffffffffu, v[q * EP + e], src);
+            if (q == 0 || piece == (unsigned)q) w[e] = x;
+          }
+        if (base + src < N) reinterpret_cast<uint4*>(A)[(unsigned long long)base * PR + r * 32 + lane] = raw;
+      }
+    }
+  } else {
+    for (unsigned id = gs_first(); id < N; id += gs_step())
+      for (int v = 0; v < nf; v++) A[(unsigned long long)id * nf + v] = (H)S[(unsigned)v * N + id];
+  }
 }
 
 }  // namespace gpumhd

@@ -85,11 +85,12 @@ struct Launch {
                             cudaStream_t s);
   static void fill_ghosts(const Consts& c, R* U, int nfield, int with_bc, cudaStream_t s);
   static void tile_state(const Geom& gd, const Geom& gs, const R* Us, R* Ud, cudaStream_t s);
-  // host cState layout (double, or float as in MURaM's SINGLE_PRECISION build) <-> device SoA
-  static void aos_to_soa(long long N, int nf, const double* A, R* S, cudaStream_t s);
-  static void soa_to_aos(long long N, int nf, const R* S, double* A, cudaStream_t s);
-  static void aos_to_soa(long long N, int nf, const float* A, R* S, cudaStream_t s);
-  static void soa_to_aos(long long N, int nf, const R* S, float* A, cudaStream_t s);
+  // host layout (double, or float as in MURaM's SINGLE_PRECISION build) <-> device
+  // arrays; host: A is pinned host memory (few blocks keep the link busy)
+  template <class H>
+  static void aos_to_soa(const Geom& g, int nf, const H* A, R* S, bool host, cudaStream_t s);
+  template <class H>
+  static void soa_to_aos(const Geom& g, int nf, const R* S, H* A, bool host, cudaStream_t s);
 };
 
 // Tile shapes of the stage kernel per state type.
@@ -465,21 +466,24 @@ void Launch<R>::fill_ghosts(const Consts& c, R* U, int nfield, int with_bc, cuda
   k_fill_ghosts<R><<<grid_for(ng, 256), 256, 0, s>>>(g, U, nfield, with_bc);
 }
 template <class R>
-void Launch<R>::aos_to_soa(long long N, int nf, const double* A, R* S, cudaStream_t s) {
-  k_aos_to_soa<R, double><<<grid_for(N, 256), 256, 0, s>>>(N, nf, A, S);
+template <class H>
+void Launch<R>::aos_to_soa(const Geom& g, int nf, const H* A, R* S, bool host, cudaStream_t s) {
+  const bool vec = nf == 8 && (uintptr_t)A % 16 == 0;
+  const int full = grid_for(g.N, 256), nb = host && full > 304 ? 304 : full;
+  (vec ? k_aos_to_soa<R, H, true> : k_aos_to_soa<R, H, false>)<<<nb, 256, 0, s>>>(g, nf, A, S);
 }
 template <class R>
-void Launch<R>::soa_to_aos(long long N, int nf, const R* S, double* A, cudaStream_t s) {
-  k_soa_to_aos<R, double><<<grid_for(N, 256), 256, 0, s>>>(N, nf, S, A);
+template <class H>
+void Launch<R>::soa_to_aos(const Geom& g, int nf, const R* S, H* A, bool host, cudaStream_t s) {
+  const bool vec = nf == 8 && (uintptr_t)A % 16 == 0;
+  const int full = grid_for(g.N, 256), nb = host && full > 304 ? 304 : full;
+  (vec ? k_soa_to_aos<R, H, true> : k_soa_to_aos<R, H, false>)<<<nb, 256, 0, s>>>(g, nf, S, A);
 }
-template <class R>
-void Launch<R>::aos_to_soa(long long N, int nf, const float* A, R* S, cudaStream_t s) {
-  k_aos_to_soa<R, float><<<grid_for(N, 256), 256, 0, s>>>(N, nf, A, S);
-}
-template <class R>
-void Launch<R>::soa_to_aos(long long N, int nf, const R* S, float* A, cudaStream_t s) {
-  k_soa_to_aos<R, float><<<grid_for(N, 256), 256, 0, s>>>(N, nf, S, A);
-}
+#define GPUMHD_CONVERSIONS(R)                                                                                  \
+  template void Launch<R>::aos_to_soa<float>(const Geom&, int, const float*, R*, bool, cudaStream_t);         \
+  template void Launch<R>::aos_to_soa<double>(const Geom&, int, const double*, R*, bool, cudaStream_t);       \
+  template void Launch<R>::soa_to_aos<float>(const Geom&, int, const R*, float*, bool, cudaStream_t);         \
+  template void Launch<R>::soa_to_aos<double>(const Geom&, int, const R*, double*, bool, cudaStream_t);
 #endif
 
 }  // namespace gpumhd

@@ -4,4 +4,5 @@
 
 namespace gpumhd {
 template struct Launch<float>;
+GPUMHD_CONVERSIONS(float)
 }  // namespace gpumhd

@@ -6,6 +6,7 @@
 namespace gpumhd {
 
 template struct Launch<double>;
+GPUMHD_CONVERSIONS(double)
 
 // The values derive_one reads.
 struct DeriveIn {

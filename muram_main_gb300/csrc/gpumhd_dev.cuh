@@ -21,7 +21,8 @@ constexpr int GH = 2;   // ghost layers
 
 struct Geom {
   int nx, ny, nz;       // interior
-  int sx, sy, sz;       // with ghosts
+  int sx, sy, sz;       // with ghosts; sx is the row pitch (FP32: nx + 4 rounded up to 16 bytes)
+  int wx;               // nodes of a row, nx + 4
   long long N;          // sx*sy*sz
   int periodic_x;
   unsigned N32;         // N as 32-bit: every offset q*N + cell of the 8 state arrays is below 2^32
@@ -321,6 +322,16 @@ __device__ __forceinline__ void interior_ijk(const Geom& g, unsigned t, int& i, 
   i = GH + (int)(t - q * nx);
   j = GH + (int)(q % ny);
   k = GH + (int)(q / ny);
+}
+// Node t of the box (x fastest, t < wx*sy*sz) -> its offset in the arrays.
+__device__ __forceinline__ unsigned node_offset(const Geom& g, unsigned t) {
+  if (g.sx == g.wx) return t;
+  const unsigned row = t / (unsigned)g.wx;
+  return t + row * (unsigned)(g.sx - g.wx);
+}
+// An element of the rows' padding (not a node).
+__device__ __forceinline__ bool is_padding(const Geom& g, unsigned id) {
+  return g.sx != g.wx && id % (unsigned)g.sx >= (unsigned)g.wx;
 }
 __device__ __forceinline__ void node_ijk(const Geom& g, unsigned id, int& i, int& j, int& k) {
   const unsigned sx = (unsigned)g.sx, sy = (unsigned)g.sy;

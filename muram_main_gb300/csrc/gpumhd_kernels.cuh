@@ -1247,7 +1247,7 @@ __global__ void __launch_bounds__(128, TvdBlocks<R>::lanes) k_tvd_sweep_xlanes(C
     const unsigned j = pen % (unsigned)g.sy, k = pen / (unsigned)g.sy;
     const long long base = (long long)g.sx * ((long long)j + (long long)g.sy * (long long)k);
     const int pos = GH + OUT * (int)seg - 2 + lane;     // this lane's cell along x
-    const int posc = min(pos, g.sx - 1);                 // clamped for the tail of the last segment
+    const int posc = min(pos, g.wx - 1);                 // clamped for the tail of the last segment
     TCell<R> c0, cl, cr, crr;
     tvd_load<R>(c, Uin, Pst, base + posc, posc, cmax_t, fac0, hyper, inv_va2max, c0);
     // from the neighbours only what the slope and the interface flux read:
@@ -1304,6 +1304,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_cons_to_prim(Consts c, 
   const Geom& g = c.g;
   const unsigned N = g.N32;
   for (unsigned id = gs_first(); id < N; id += gs_step()) {
+    if (is_padding(g, id)) continue;
     R d = U[id];
     R v1, v2, v3, ei;
     prim_from_cons(d, U[N + id], U[2 * N + id], U[3 * N + id], U[4 * N + id], v1, v2, v3, ei);
@@ -1333,6 +1334,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_aux_of_snapshot(Consts 
                                                                     R* __restrict__ Ri, R* __restrict__ Am) {
   const unsigned N = c.g.N32;
   for (unsigned id = gs_first(); id < N; id += gs_step()) {
+    if (is_padding(c.g, id)) continue;
     const R d = T[id], ei = Ne[id];
     const R dn = d_div((R)1.0, d);
     R pr, tm, ne, ri, am;
@@ -1352,6 +1354,7 @@ __global__ void k_init_pass(Consts c, const R* __restrict__ U, R* __restrict__ P
   const R vlim95 = dynr<R>(dyn).vlim95, elim95 = dynr<R>(dyn).elim95;
   const unsigned N = g.N32;
   for (unsigned id = gs_first(); id < N; id += gs_step()) {
+    if (is_padding(g, id)) continue;
     R d = U[id];
     R v1, v2, v3, ei;
     prim_from_cons(d, U[N + id], U[2 * N + id], U[3 * N + id], U[4 * N + id], v1, v2, v3, ei);
@@ -1671,7 +1674,7 @@ __global__ void k_fill_ghosts(Geom g, R* __restrict__ U, int nfield, int with_bc
   const unsigned N = g.N32;
   // the ghost nodes only, in three x-fastest groups: the z-ghost planes, the
   // y-ghost rows of interior planes, the x-ghost nodes of interior rows
-  const unsigned sx = (unsigned)g.sx, sy = (unsigned)g.sy;
+  const unsigned sx = (unsigned)g.wx, sy = (unsigned)g.sy;
   const unsigned nA = 2u * GH * sx * sy;
   const unsigned nB = 2u * GH * sx * (unsigned)g.nz;
   const unsigned nC = 2u * GH * (unsigned)g.ny * (unsigned)g.nz;
@@ -1723,8 +1726,9 @@ __global__ void k_fill_ghosts(Geom g, R* __restrict__ U, int nfield, int with_bc
 // covers 512 contiguous bytes (one record per thread instead: 8 ms).
 template <class R, class H, bool VEC>
 __global__ void k_aos_to_soa(Geom g, int nf, const H* __restrict__ A, R* __restrict__ S) {
-  const unsigned N = g.N32;
-  for (unsigned id = gs_first(); id < N; id += gs_step()) {
+  const unsigned N = g.N32, n = (unsigned)g.wx * (unsigned)g.sy * (unsigned)g.sz;
+  for (unsigned id = gs_first(); id < n; id += gs_step()) {
+    const unsigned o = node_offset(g, id);
     if constexpr (VEC) {
       constexpr int PR = 8 * sizeof(H) / 16, EP = 16 / sizeof(H);  // 16-byte pieces per record, values per piece
       uint4 raw[PR];
@@ -1733,20 +1737,20 @@ __global__ void k_aos_to_soa(Geom g, int nf, const H* __restrict__ A, R* __restr
       for (int q = 0; q < PR; q++) raw[q] = p[q];
       const H* v = reinterpret_cast<const H*>(raw);
 #pragma unroll
-      for (int q = 0; q < PR * EP; q++) S[(unsigned)q * N + id] = (R)v[q];
+      for (int q = 0; q < PR * EP; q++) S[(unsigned)q * N + o] = (R)v[q];
     } else {
-      for (int v = 0; v < nf; v++) S[(unsigned)v * N + id] = (R)A[(unsigned long long)id * nf + v];
+      for (int v = 0; v < nf; v++) S[(unsigned)v * N + o] = (R)A[(unsigned long long)id * nf + v];
     }
   }
 }
 template <class R, class H, bool VEC>
 __global__ void k_soa_to_aos(Geom g, int nf, const R* __restrict__ S, H* __restrict__ A) {
-  const unsigned N = g.N32;
+  const unsigned N = g.N32, n = (unsigned)g.wx * (unsigned)g.sy * (unsigned)g.sz;
   if constexpr (VEC) {
     constexpr int PR = 8 * sizeof(H) / 16, EP = 16 / sizeof(H), RW = 32 / PR;  // records per warp store
     const unsigned lane = threadIdx.x & 31u;
-    for (unsigned base = gs_first() - lane; base < N; base += gs_step()) {
-      const unsigned id = min(base + lane, N - 1u);
+    for (unsigned base = gs_first() - lane; base < n; base += gs_step()) {
+      const unsigned id = node_offset(g, min(base + lane, n - 1u));
       H v[8];
 #pragma unroll
       for (int q = 0; q < 8; q++) v[q] = (H)S[(unsigned)q * N + id];
@@ -1762,12 +1766,14 @@ __global__ void k_soa_to_aos(Geom g, int nf, const R* __restrict__ S, H* __restr
             const H x = __shfl_sync(0xffffffffu, v[q * EP + e], src);
             if (q == 0 || piece == (unsigned)q) w[e] = x;
           }
-        if (base + src < N) reinterpret_cast<uint4*>(A)[(unsigned long long)base * PR + r * 32 + lane] = raw;
+        if (base + src < n) reinterpret_cast<uint4*>(A)[(unsigned long long)base * PR + r * 32 + lane] = raw;
       }
     }
   } else {
-    for (unsigned id = gs_first(); id < N; id += gs_step())
-      for (int v = 0; v < nf; v++) A[(unsigned long long)id * nf + v] = (H)S[(unsigned)v * N + id];
+    for (unsigned id = gs_first(); id < n; id += gs_step()) {
+      const unsigned o = node_offset(g, id);
+      for (int v = 0; v < nf; v++) A[(unsigned long long)id * nf + v] = (H)S[(unsigned)v * N + o];
+    }
   }
 }
 

@@ -462,7 +462,7 @@ void Launch<R>::tile_state(const Geom& gd, const Geom& gs, const R* Us, R* Ud, c
 template <class R>
 void Launch<R>::fill_ghosts(const Consts& c, R* U, int nfield, int with_bc, cudaStream_t s) {
   const Geom& g = c.g;
-  const long long ng = 2LL * GH * ((long long)g.sx * g.sy + (long long)g.sx * g.nz + (long long)g.ny * g.nz);
+  const long long ng = 2LL * GH * ((long long)g.wx * g.sy + (long long)g.wx * g.nz + (long long)g.ny * g.nz);
   k_fill_ghosts<R><<<grid_for(ng, 256), 256, 0, s>>>(g, U, nfield, with_bc);
 }
 template <class R>

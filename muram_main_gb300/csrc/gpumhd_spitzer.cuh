@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_temp(Consts c, const R*
   const Geom& g = c.g;
   const unsigned N = g.N32;
   for (unsigned id = gs_first(); id < N; id += gs_step()) {
+    if (is_padding(g, id)) continue;
     R v1, v2, v3, ei;
     const R d = U[id];
     prim_from_cons(d, U[N + id], U[2 * N + id], U[3 * N + id], U[4 * N + id], v1, v2, v3, ei);

@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, 
   const unsigned seg = warp % nseg, pen0 = warp / nseg;
   if (pen0 >= stride) return;
   const int pos = OUT * (int)seg + lane;   // this lane's cell along x (the first is GH - 2)
-  const int posc = min(pos, g.sx - 1);     // clamped for the tail of the last segment
+  const int posc = min(pos, g.wx - 1);     // clamped for the tail of the last segment
   const bool out = lane >= 2 && lane < 30 && pos < GH + g.nx;
   const Prof pr = prof_of(k, posc);
   const Sweep s = sweep_of(dyn->rf, k, 0);

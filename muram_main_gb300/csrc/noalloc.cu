@@ -96,7 +96,7 @@ extern "C" int gpumhd_cfl_dt_noalloc(const double* U_prim, const double* pres, i
   }
   Geom g;
   g.nx = nx; g.ny = ny; g.nz = nz;
-  g.sx = nx + 2 * GH; g.sy = ny + 2 * GH; g.sz = nz + 2 * GH;
+  g.sx = g.wx = nx + 2 * GH; g.sy = ny + 2 * GH; g.sz = nz + 2 * GH;
   g.N = (long long)g.sx * g.sy * g.sz;
   g.periodic_x = 1;
   g.N32 = (unsigned)g.N;

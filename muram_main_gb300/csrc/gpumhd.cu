@@ -16,6 +16,14 @@
 
 using namespace gpumhd;
 
+// Pinned landing place of the step-control block and a run's time steps, so
+// that a call copies them in stream order and waits once.
+constexpr int PIN_HIST = 1024;
+struct PinnedBack {
+  Dyn dyn;
+  double hist[PIN_HIST];
+};
+
 struct gpumhd_ctx {
   gpumhd_params p;
   int device = 0;
@@ -45,6 +53,7 @@ struct gpumhd_ctx {
   double* dt_hist = nullptr;
   int dt_hist_cap = 0;
   Dyn hdyn{};                                  // host mirror of the per-routine scalars
+  PinnedBack* pin = nullptr;
   // EOS
   double* d_xeps = nullptr;
   double* d_xlr = nullptr;
@@ -368,8 +377,9 @@ static int push_dyn(gpumhd_ctx* ctx) {
   return GPUMHD_OK;
 }
 static int pull_dyn(gpumhd_ctx* ctx) {
-  CK(cudaMemcpyAsync(&ctx->hdyn, ctx->dyn, sizeof(Dyn), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(&ctx->pin->dyn, ctx->dyn, sizeof(Dyn), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->hdyn = ctx->pin->dyn;
   return GPUMHD_OK;
 }
 
@@ -471,6 +481,7 @@ extern "C" int gpumhd_create(const gpumhd_params* p, int device, gpumhd_ctx** ou
       if (cudaMalloc(&ctx->P[b], N * ctx->rsz) != cudaSuccess) { rc = GPUMHD_E_NOMEM; break; }
     if (rc) break;
     if (cudaMalloc(&ctx->dyn, sizeof(Dyn)) != cudaSuccess) { rc = GPUMHD_E_NOMEM; break; }
+    if (cudaMallocHost(&ctx->pin, sizeof(PinnedBack)) != cudaSuccess) { rc = GPUMHD_E_NOMEM; break; }
     ctx->tma = ctx->f32 ? make_tensor_maps<float>(ctx) : make_tensor_maps<double>(ctx);
     for (int b = 0; b < 3; b++) cudaMemsetAsync(ctx->S[b], 0, 8 * N * ctx->rsz, ctx->stream);
     for (int b = 0; b < 2; b++) cudaMemsetAsync(ctx->P[b], 0, N * ctx->rsz, ctx->stream);
@@ -530,6 +541,7 @@ extern "C" int gpumhd_destroy(gpumhd_ctx* ctx) {
   for (void* q : ctx->spt) cudaFree(q);
   cudaFree(ctx->d_d3); cudaFree(ctx->d_eps3);
   cudaFree(ctx->dyn);
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   cudaFree(ctx->dt_hist);
   cudaFree(ctx->d_xeps);
   cudaFree(ctx->d_xlr);
@@ -1725,11 +1737,10 @@ static int capture_graph(gpumhd_ctx* ctx) {
 extern "C" int gpumhd_synchronize(gpumhd_ctx* ctx) {
   if (!ctx) return GPUMHD_E_INVALID;
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamSynchronize(ctx->stream));
+  int rc = pull_dyn(ctx);  // waits for the stream
+  if (rc) return rc;
   if (ctx->s_out) CK(cudaStreamSynchronize(ctx->s_out));
   if (ctx->s_in) CK(cudaStreamSynchronize(ctx->s_in));
-  int rc = pull_dyn(ctx);
-  if (rc) return rc;
   switch (ctx->hdyn.err) {
     case 0: return GPUMHD_OK;
     case ERR_BAD_DT_RAD: return fail(ctx, GPUMHD_E_BAD_DT, "Invalid time step: dt_rad");
@@ -1747,17 +1758,20 @@ extern "C" int gpumhd_run_steps(gpumhd_ctx* ctx, int nsteps, double* dt_out, int
   if (rc) return rc;
   // dt history restarts at this call
   ctx->hdyn.steps_done = 0;
-  CK(cudaMemcpyAsync(&ctx->dyn->steps_done, &ctx->hdyn.steps_done, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemsetAsync(&ctx->dyn->steps_done, 0, sizeof(int), ctx->stream));
   if (capture) {
     rc = capture_graph(ctx);
     if (rc) return rc;
   }
   rc = gpumhd_enqueue_steps(ctx, nsteps);
   if (rc) return rc;
+  const bool hist = dt_out && nsteps > 0, pinned = hist && nsteps <= PIN_HIST;
+  if (pinned)
+    CK(cudaMemcpyAsync(ctx->pin->hist, ctx->dt_hist, sizeof(double) * nsteps, cudaMemcpyDeviceToHost, ctx->stream));
   rc = gpumhd_synchronize(ctx);
   if (rc) return rc;
-  if (dt_out && nsteps > 0)
-    CK(cudaMemcpy(dt_out, ctx->dt_hist, sizeof(double) * nsteps, cudaMemcpyDeviceToHost));
+  if (pinned) memcpy(dt_out, ctx->pin->hist, sizeof(double) * nsteps);
+  else if (hist) CK(cudaMemcpy(dt_out, ctx->dt_hist, sizeof(double) * nsteps, cudaMemcpyDeviceToHost));
   return GPUMHD_OK;
 }
 

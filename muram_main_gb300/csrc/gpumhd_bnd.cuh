@@ -34,51 +34,43 @@ constexpr int BND_SETUP_THREADS = 256;
 
 // Axes x0 + del*i as eos_init stores them (src/eos_init.C:125-146).
 __device__ __forceinline__ void bnd_w(double x, double x0, double del, int i, double& lo, double& hi) {
-  lo = x - (x0 + del * ((double)i));
-  hi = (x0 + del * ((double)(i + 1))) - x;
+  lo = x - (x0 + del * i64f::from_float((float)i));  // i < 2^24: exact
+  hi = (x0 + del * i64f::from_float((float)(i + 1))) - x;
 }
 
 // p_interp / s_interp (src/eos_init.C:268-343): ln p or s + ss_off
 __device__ __forceinline__ double bnd_fwd(const Consts& c, const float* T, double ee, double dd) {
   const BndK<double>& b = c.bndd;
-  const double ee1 = log(ee + b.eps_off);
-  const double logr = log(dd);
-  int i = cvt_x86((ee1 - b.eps0) * b.inv_del_eps);
-  if (i < 0) i = 0;
-  if (i > c.N_eps - 2) i = c.N_eps - 2;
-  int j = cvt_x86((logr - b.lr0) * b.inv_del_lr);
-  if (j < 0) j = 0;
-  if (j > c.N_lr - 2) j = c.N_lr - 2;
+  const double ee1 = d_log(ee + b.eps_off);
+  const double logr = d_log(dd);
+  const int i = min(i64f::trunc_pos((ee1 - b.eps0) * b.inv_del_eps), c.N_eps - 2);
+  const int j = min(i64f::trunc_pos((logr - b.lr0) * b.inv_del_lr), c.N_lr - 2);
   double we0, we1, wr0, wr1;
   bnd_w(ee1, b.eps0, b.del_eps, i, we0, we1);
   bnd_w(logr, b.lr0, b.del_lr, j, wr0, wr1);
   const long long L = c.N_lr;
-  return wr0 * we0 * (double)T[(i + 1) * L + j + 1] + wr0 * we1 * (double)T[i * L + j + 1] +
-         wr1 * we0 * (double)T[(i + 1) * L + j] + wr1 * we1 * (double)T[i * L + j];
+  return wr0 * we0 * i64f::from_float(T[(i + 1) * L + j + 1]) + wr0 * we1 * i64f::from_float(T[i * L + j + 1]) +
+         wr1 * we0 * i64f::from_float(T[(i + 1) * L + j]) + wr1 * we1 * i64f::from_float(T[i * L + j]);
 }
 // The same two lookups as bnd_fwd on two tables (ln p and s + ss_off) at one
 // (ee, dd): logs, cell and weights formed once, each sum as bnd_fwd's.
 __device__ __forceinline__ void bnd_fwd2(const Consts& c, const float* T1, const float* T2, double ee, double dd,
                                          double& o1, double& o2) {
   const BndK<double>& b = c.bndd;
-  const double ee1 = log(ee + b.eps_off);
-  const double logr = log(dd);
-  int i = cvt_x86((ee1 - b.eps0) * b.inv_del_eps);
-  if (i < 0) i = 0;
-  if (i > c.N_eps - 2) i = c.N_eps - 2;
-  int j = cvt_x86((logr - b.lr0) * b.inv_del_lr);
-  if (j < 0) j = 0;
-  if (j > c.N_lr - 2) j = c.N_lr - 2;
+  const double ee1 = d_log(ee + b.eps_off);
+  const double logr = d_log(dd);
+  const int i = min(i64f::trunc_pos((ee1 - b.eps0) * b.inv_del_eps), c.N_eps - 2);
+  const int j = min(i64f::trunc_pos((logr - b.lr0) * b.inv_del_lr), c.N_lr - 2);
   double we0, we1, wr0, wr1;
   bnd_w(ee1, b.eps0, b.del_eps, i, we0, we1);
   bnd_w(logr, b.lr0, b.del_lr, j, wr0, wr1);
   const long long L = c.N_lr;
-  o1 = wr0 * we0 * (double)T1[(i + 1) * L + j + 1] + wr0 * we1 * (double)T1[i * L + j + 1] +
-       wr1 * we0 * (double)T1[(i + 1) * L + j] + wr1 * we1 * (double)T1[i * L + j];
-  o2 = wr0 * we0 * (double)T2[(i + 1) * L + j + 1] + wr0 * we1 * (double)T2[i * L + j + 1] +
-       wr1 * we0 * (double)T2[(i + 1) * L + j] + wr1 * we1 * (double)T2[i * L + j];
+  o1 = wr0 * we0 * i64f::from_float(T1[(i + 1) * L + j + 1]) + wr0 * we1 * i64f::from_float(T1[i * L + j + 1]) +
+       wr1 * we0 * i64f::from_float(T1[(i + 1) * L + j]) + wr1 * we1 * i64f::from_float(T1[i * L + j]);
+  o2 = wr0 * we0 * i64f::from_float(T2[(i + 1) * L + j + 1]) + wr0 * we1 * i64f::from_float(T2[i * L + j + 1]) +
+       wr1 * we0 * i64f::from_float(T2[(i + 1) * L + j]) + wr1 * we1 * i64f::from_float(T2[i * L + j]);
 }
-__device__ __forceinline__ double bnd_p(const Consts& c, double ee, double dd) { return exp(bnd_fwd(c, c.tab[0], ee, dd)); }
+__device__ __forceinline__ double bnd_p(const Consts& c, double ee, double dd) { return d_exp(bnd_fwd(c, c.tab[0], ee, dd)); }
 __device__ __forceinline__ double bnd_s(const Consts& c, double ee, double dd) {
   return bnd_fwd(c, c.tab[2], ee, dd) - c.bndd.ss_off;
 }
@@ -87,23 +79,19 @@ __device__ __forceinline__ double bnd_s(const Consts& c, double ee, double dd) {
 __device__ __forceinline__ void bnd_inv2(const Consts& c, double pp, double ss, double& lrho, double& leps) {
   const BndK<double>& b = c.bndd;
   const double ss1 = ss + b.ss_off;
-  const double logp = log(pp);
-  int i = cvt_x86((logp - b.lp30) * b.inv_del_lp3);
-  if (i < 0) i = 0;
-  if (i > c.N_lp3 - 2) i = c.N_lp3 - 2;
-  int j = cvt_x86((ss1 - b.s30) * b.inv_del_s3);
-  if (j < 0) j = 0;
-  if (j > c.N_s3 - 2) j = c.N_s3 - 2;
+  const double logp = d_log(pp);
+  const int i = min(i64f::trunc_pos((logp - b.lp30) * b.inv_del_lp3), c.N_lp3 - 2);
+  const int j = min(i64f::trunc_pos((ss1 - b.s30) * b.inv_del_s3), c.N_s3 - 2);
   double wp0, wp1, ws0, ws1;
   bnd_w(logp, b.lp30, b.del_lp3, i, wp0, wp1);
   bnd_w(ss1, b.s30, b.del_s3, j, ws0, ws1);
   const long long L = c.N_s3;
   const float* D = c.d3;
   const float* E = c.eps3;
-  lrho = wp0 * ws0 * (double)D[(i + 1) * L + j + 1] + wp0 * ws1 * (double)D[(i + 1) * L + j] +
-         wp1 * ws0 * (double)D[i * L + j + 1] + wp1 * ws1 * (double)D[i * L + j];
-  leps = wp0 * ws0 * (double)E[(i + 1) * L + j + 1] + wp0 * ws1 * (double)E[(i + 1) * L + j] +
-         wp1 * ws0 * (double)E[i * L + j + 1] + wp1 * ws1 * (double)E[i * L + j];
+  lrho = wp0 * ws0 * i64f::from_float(D[(i + 1) * L + j + 1]) + wp0 * ws1 * i64f::from_float(D[(i + 1) * L + j]) +
+         wp1 * ws0 * i64f::from_float(D[i * L + j + 1]) + wp1 * ws1 * i64f::from_float(D[i * L + j]);
+  leps = wp0 * ws0 * i64f::from_float(E[(i + 1) * L + j + 1]) + wp0 * ws1 * i64f::from_float(E[(i + 1) * L + j]) +
+         wp1 * ws0 * i64f::from_float(E[i * L + j + 1]) + wp1 * ws1 * i64f::from_float(E[i * L + j]);
 }
 
 // Per block of 32 (y) x 4 (z) interior columns: sums over the first two
@@ -128,9 +116,9 @@ __global__ void __launch_bounds__(BND_THREADS) k_bc_sums(Consts c, const R* __re
     const double n1 = (double)U[g.N + c2], n2 = (double)U[2 * g.N + c2], n3 = (double)U[3 * g.N + c2];
     const double e1 = (double)U[4 * g.N + c1], e2 = (double)U[4 * g.N + c2];
     const double mm1 = m1 * m1 + m2 * m2 + m3 * m3, mm2 = n1 * n1 + n2 * n2 + n3 * n3;
-    const double ea1 = e1 - 0.5 * (mm1 / d1), ea2 = e2 - 0.5 * (mm2 / d2);
-    q[0] = bnd_p(c, ea1 / d1, d1);
-    q[1] = bnd_p(c, ea2 / d2, d2);
+    const double ea1 = e1 - d_half(d_div(mm1, d1)), ea2 = e2 - d_half(d_div(mm2, d2));
+    q[0] = bnd_p(c, d_div(ea1, d1), d1);
+    q[1] = bnd_p(c, d_div(ea2, d2), d2);
     if (ini) {
       const double eb1 = e1 - 0.5 * mm1 / d1, eb2 = e2 - 0.5 * mm2 / d2;
       q[2] = bnd_p(c, eb1 / d1, d1);
@@ -191,7 +179,7 @@ __global__ void __launch_bounds__(BND_THREADS) k_bc_ghosts(Consts c, R* __restri
       if (P || cm_col) {
         R v1, v2, v3, ei;
         prim_from_cons(w[0], w[1], w[2], w[3], w[4], v1, v2, v3, ei);
-        const R pr = eos_pres(c, w[0], ei, (R)1.0 / w[0]);
+        const R pr = eos_pres(c, w[0], ei, d_div((R)1.0, w[0]));
         if (P) P[id] = pr;
         if (cm_col) cm = smax(cm, cmax_cell<R>(w[0], v1, v2, v3, w[5], w[6], w[7], pr, dynr<R>(dyn).inv_va2max));
       }
@@ -207,14 +195,14 @@ __global__ void __launch_bounds__(BND_THREADS) k_bc_ghosts(Consts c, R* __restri
       // bottom (src/boundary_pdmp_1_fftw3.C:227-310)
       const double p1_dmp = 0.8;
       const double pmean1 = dyn->pmean1, pmean2 = dyn->pmean2, p_bc = dyn->p_bc, s_bc = dyn->s_bc;
-      u1[4] -= 0.5 * (u1[1] * u1[1] + u1[2] * u1[2] + u1[3] * u1[3]) / u1[0];
-      u2[4] -= 0.5 * (u2[1] * u2[1] + u2[2] * u2[2] + u2[3] * u2[3]) / u2[0];
-      double eps1 = u1[4] / u1[0], eps2 = u2[4] / u2[0];
-      const double pmag = 0.5 * u1[5] * u1[5];
+      u1[4] -= d_div(d_half(u1[1] * u1[1] + u1[2] * u1[2] + u1[3] * u1[3]), u1[0]);
+      u2[4] -= d_div(d_half(u2[1] * u2[1] + u2[2] * u2[2] + u2[3] * u2[3]), u2[0]);
+      double eps1 = d_div(u1[4], u1[0]), eps2 = d_div(u2[4], u2[0]);
+      const double pmag = d_half(u1[5]) * u1[5];
       // p_interp and s_interp of the first layer share their logs and weights
       double lnp1, ss1;
       bnd_fwd2(c, c.tab[0], c.tab[2], eps1, u1[0], lnp1, ss1);
-      const double pmin1 = exp(lnp1) - pmean1;
+      const double pmin1 = d_exp(lnp1) - pmean1;
       double s1, s2;
       if (u1[1] >= 0.e0) {
         s1 = s_bc;
@@ -223,16 +211,16 @@ __global__ void __launch_bounds__(BND_THREADS) k_bc_ghosts(Consts c, R* __restri
         s1 = ss1 - c.bndd.ss_off;
         s2 = bnd_s(c, eps2, u2[0]);
       }
-      double cc = p_bc / sqrt(pmean1 * pmean2);
+      double cc = d_div(p_bc, d_sqrt(pmean1 * pmean2));
       double p1 = pmean1 * cc;
       double p2 = pmean1 * cc * cc;
       p1 += pmin1 * p1_dmp;
       p2 += pmin1 * p1_dmp * p1_dmp;
       p1 -= pmag * (1.0 - p1_dmp);
       p2 -= pmag * (1.0 - p1_dmp * p1_dmp);
-      cc = u1[5] / b.bcrit;
+      cc = d_div(u1[5], b.bcrit);
       cc = (cc * cc) * (cc * cc);  // pow(cc, 4) to the last bit or two
-      cc = (1.0 - cc) / (1.0 + cc);
+      cc = d_div(1.0 - cc, 1.0 + cc);
 #pragma unroll
       for (int v = 1; v <= 3; v++) {
         u1[v] *= cc;
@@ -241,13 +229,13 @@ __global__ void __launch_bounds__(BND_THREADS) k_bc_ghosts(Consts c, R* __restri
       double lr1, le1, lr2, le2;
       bnd_inv2(c, p1, s1, lr1, le1);
       bnd_inv2(c, p2, s2, lr2, le2);
-      const double rho1 = exp(lr1), rho2 = exp(lr2);
-      eps1 = exp(le1) - b.eps_off;
-      eps2 = exp(le2) - b.eps_off;
+      const double rho1 = d_exp(lr1), rho2 = d_exp(lr2);
+      eps1 = d_exp(le1) - b.eps_off;
+      eps2 = d_exp(le2) - b.eps_off;
       u1[0] = rho1;
       u2[0] = rho2;
-      u1[4] = eps1 * rho1 + 0.5 * (u1[1] * u1[1] + u1[2] * u1[2] + u1[3] * u1[3]) / u1[0];
-      u2[4] = eps2 * rho2 + 0.5 * (u2[1] * u2[1] + u2[2] * u2[2] + u2[3] * u2[3]) / u2[0];
+      u1[4] = eps1 * rho1 + d_div(d_half(u1[1] * u1[1] + u1[2] * u1[2] + u1[3] * u1[3]), u1[0]);
+      u2[4] = eps2 * rho2 + d_div(d_half(u2[1] * u2[1] + u2[2] * u2[2] + u2[3] * u2[3]), u2[0]);
       out(lb - 1, u1);
       out(lb - 2, u2);
       if (sflx) {  // heat flux: zero in the bottom ghosts (src/boundary_pdmp_1_fftw3.C:302-306)

@@ -3,8 +3,8 @@
 Five translation units are compiled in parallel and linked into
 ``muram_main_gb300/_build/libgpumhd.so``:
 
-* ``kernels_f64.cu`` with ``--fmad=false`` (every product and sum rounds
-  separately, like the reference's no-FMA builds);
+* ``kernels_f64.cu`` with ``--fmad=false`` (the compiler contracts nothing: the
+  sources say where a product and a sum round once);
 * ``kernels_f32.cu`` with FMA contraction;
 * ``gpumhd.cu`` (host side of the C ABI), host code with -ffp-contract=off;
 * ``adjoint.cu`` (the FP64 adjoint kernels) and ``noalloc.cu`` (the
@@ -53,7 +53,8 @@ def build(force=False, verbose=False):
     common = [nvcc, "-std=c++17", ARCH, "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
               "-I", INCLUDE, "-c"]
     # FP32: contraction, approximate division and square root (within the
-    # FP32 mode's error budget); FP64: every operation IEEE-rounded.
+    # FP32 mode's error budget); FP64: every operation IEEE-rounded, fused
+    # multiply-adds only where written.
     units = [("kernels_f64.cu", ["--fmad=false"]),
              ("kernels_f32.cu", ["--fmad=true", "-prec-div=false", "-prec-sqrt=false"]),
              ("gpumhd.cu", ["--fmad=false"]),

@@ -279,7 +279,7 @@ __global__ void k_stage_a(Consts c, const Dyn* dyn, Box b, const double* __restr
         else if (d == 1) flux12<double, 1>(w, 1, f[s], 1);
         else flux12<double, 2>(w, 1, f[s], 1);
       }
-      for (int q = 0; q < NF; q++) Dq[d][q] = k.w1[d] * (f[2][q] - f[1][q]) + k.w2[d] * (f[3][q] - f[0][q]);
+      for (int q = 0; q < NF; q++) Dq[d][q] = mad(k.w1[d], f[2][q] - f[1][q], k.w2[d] * (f[3][q] - f[0][q]));
     }
     const double lf = boris_lf<double>(cen, inv_va2max);
     double R[NV];

@@ -167,8 +167,8 @@ __device__ __forceinline__ void prim_from_cons(R d, R m1, R m2, R m3, R e, R& v1
   v1 = m1 * dn;
   v2 = m2 * dn;
   v3 = m3 * dn;
-  R vv = v1 * v1 + v2 * v2 + v3 * v3;
-  ei = e - d_half(vv) * d;
+  R vv = dot3(v1, v1, v2, v2, v3, v3);
+  ei = nmad(d_half(vv), d, e);
 }
 
 // The 9 stored values of a cell (state and pressure), as loaded from memory.
@@ -210,8 +210,8 @@ __device__ __forceinline__ void prim_of_raw(const Raw9<R>& r, R* out) {
   R v1, v2, v3, ei;
   if (PRIM_IN) { v1 = a1; v2 = a2; v3 = a3; ei = a4; }
   else prim_from_cons(d, a1, a2, a3, a4, v1, v2, v3, ei);
-  R vv = v1 * v1 + v2 * v2 + v3 * v3;
-  R bb = b1 * b1 + b2 * b2 + b3 * b3;
+  R vv = dot3(v1, v1, v2, v2, v3, v3);
+  R bb = dot3(b1, b1, b2, b2, b3, b3);
   out[P_D] = d;
   out[P_V1] = v1;
   out[P_V2] = v2;
@@ -244,18 +244,16 @@ __device__ __forceinline__ void flux12(const R* p, int s, R* f, int fs) {
   const R mag = D1 == 0 ? b1 : (D1 == 1 ? b2 : b3);
   const R mflx = vel * d;
   f[0 * fs] = mflx;
-  f[1 * fs] = mflx * v1;
-  f[2 * fs] = mflx * v2;
-  f[3 * fs] = mflx * v3;
-  f[(1 + D1) * fs] += pr;
+  f[1 * fs] = D1 == 0 ? mad(mflx, v1, pr) : mflx * v1;
+  f[2 * fs] = D1 == 1 ? mad(mflx, v2, pr) : mflx * v2;
+  f[3 * fs] = D1 == 2 ? mad(mflx, v3, pr) : mflx * v3;
   f[4 * fs] = vel * (ei + ekin + pr);
-  const R F5 = vel * b1 - v1 * mag, F6 = vel * b2 - v2 * mag, F7 = vel * b3 - v3 * mag;
+  const R F5 = nmad(v1, mag, vel * b1), F6 = nmad(v2, mag, vel * b2), F7 = nmad(v3, mag, vel * b3);
   f[5 * fs] = Dirs<D1>::fa == 5 ? F5 : F6;
   f[6 * fs] = Dirs<D1>::fb == 7 ? F7 : F6;
-  f[7 * fs] = mag * b1;
-  f[8 * fs] = mag * b2;
-  f[9 * fs] = mag * b3;
-  f[(7 + D1) * fs] -= pmag;
+  f[7 * fs] = D1 == 0 ? mad(mag, b1, -pmag) : mag * b1;
+  f[8 * fs] = D1 == 1 ? mad(mag, b2, -pmag) : mag * b2;
+  f[9 * fs] = D1 == 2 ? mad(mag, b3, -pmag) : mag * b3;
   f[10 * fs] = Dirs<D1>::d2 == 0 ? b1 : b2;
   f[11 * fs] = Dirs<D1>::d3 == 1 ? b2 : b3;
 }
@@ -266,7 +264,7 @@ __device__ __forceinline__ void flux12(const R* p, int s, R* f, int fs) {
 __device__ __forceinline__ void deriv12(double* Dq, const double* fm2, const double* fm1, const double* fp1,
                                         const double* fp2, double w1, double w2) {
 #pragma unroll
-  for (int q = 0; q < NF; q++) Dq[q] = w1 * (fp1[q] - fm1[q]) + w2 * (fp2[q] - fm2[q]);
+  for (int q = 0; q < NF; q++) Dq[q] = mad(w1, fp1[q] - fm1[q], w2 * (fp2[q] - fm2[q]));
 }
 __device__ __forceinline__ void deriv12(float* Dq, const float* fm2, const float* fm1, const float* fp1,
                                         const float* fp2, float w1, float w2) {
@@ -294,19 +292,20 @@ __device__ __forceinline__ void apply_direction(R* Racc, const R* Dq, const R* c
   const R Bd1 = cen[P_B1 + D1];
   const R Bd2 = cen[P_B1 + Dirs<D1>::d2], Bd3 = cen[P_B1 + Dirs<D1>::d3];
   R cbb[3];
-  cbb[D1] = -Bd2 * dB2 - Bd3 * dB3;
+  cbb[D1] = nmad(Bd3, dB3, -Bd2 * dB2);
   cbb[Dirs<D1>::d2] = Bd1 * dB2;
   cbb[Dirs<D1>::d3] = Bd1 * dB3;
-  const R lrt0 = lf * Dq[7] + ((R)1.0 - lf) * cbb[0];
-  const R lrt1 = lf * Dq[8] + ((R)1.0 - lf) * cbb[1];
-  const R lrt2 = lf * Dq[9] + ((R)1.0 - lf) * cbb[2];
+  const R lc = (R)1.0 - lf;
+  const R lrt0 = mad(lf, Dq[7], lc * cbb[0]);
+  const R lrt1 = mad(lf, Dq[8], lc * cbb[1]);
+  const R lrt2 = mad(lf, Dq[9], lc * cbb[2]);
   // Racc += (0 - D(F)) + Lorentz terms; FIRST: Racc is zero and not read
   R res[NV];
   res[0] = -Dq[0];
   res[1] = lrt0 - Dq[1];
   res[2] = lrt1 - Dq[2];
   res[3] = lrt2 - Dq[3];
-  res[4] = (cen[P_V1] * lrt0 + cen[P_V2] * lrt1 + cen[P_V3] * lrt2) - Dq[4];
+  res[4] = dot3(cen[P_V1], lrt0, cen[P_V2], lrt1, cen[P_V3], lrt2) - Dq[4];
   res[5 + D1] = (R)0.0;
   res[Dirs<D1>::fa] = -Dq[5];
   res[Dirs<D1>::fb] = -Dq[6];
@@ -395,7 +394,7 @@ __device__ __forceinline__ void rk_update(const Consts& c, Rem<R>* __restrict__ 
                                           const R* base, const R* Racc, R vmax, R emax, R* un) {
   if (Cc == nullptr) {
 #pragma unroll
-    for (int v = 0; v < NV; v++) un[v] = base[v] + wdt * Racc[v];
+    for (int v = 0; v < NV; v++) un[v] = mad(wdt, Racc[v], base[v]);
     tcheck_cell<R>(c, vmax, emax, un[0], un[1], un[2], un[3], un[4]);
     return;
   }
@@ -419,10 +418,10 @@ __device__ __forceinline__ void rk_update(const Consts& c, Rem<R>* __restrict__ 
 template <class R>
 __device__ __forceinline__ R boris_lf(const R* cen, R inv_va2max) {
   const R dn = d_div((R)1.0, cen[P_D]);
-  const R bb = cen[P_B1] * cen[P_B1] + cen[P_B2] * cen[P_B2] + cen[P_B3] * cen[P_B3];
+  const R bb = dot3(cen[P_B1], cen[P_B1], cen[P_B2], cen[P_B2], cen[P_B3], cen[P_B3]);
   const R va2 = bb * dn;
-  const R x2 = va2 * inv_va2max, x4 = x2 * x2, s = (R)1.0 + x2;
-  return d_div(s, s + x4);
+  const R x2 = va2 * inv_va2max, s = (R)1.0 + x2;
+  return d_div(s, mad(x2, x2, s));
 }
 
 // Sources and semi-relativistic (Boris) correction added to the residual Racc
@@ -443,16 +442,16 @@ __device__ __forceinline__ void stage_sources(R* Racc, const R* cen, R gx, R inv
   if (!rad_ok) Racc[4] = (R)NAN;
   const R rd = Racc[0];
   R fx = Racc[1], fy = Racc[2], fz = Racc[3];
-  const R bb = bx * bx + by * by + bz * bz;
+  const R bb = dot3(bx, bx, by, by, bz, bz);
   const R va2 = d_div(bb, rh);
   const R x2 = va2 * inv_va2max, x4 = x2 * x2;
   const R bf = d_div(x4, (R)1 + x2 + x4);
-  fx -= vx * rd;
-  fy -= vy * rd;
-  fz -= vz * rd;
-  const R q = d_div(fx * bx + fy * by + fz * bz, d_fmax(tiny100<R>(), bb));
-  const R b0 = -bf * (fx - q * bx), b1 = -bf * (fy - q * by), b2 = -bf * (fz - q * bz);
-  const R b3 = b0 * vx + b1 * vy + b2 * vz;
+  fx = nmad(vx, rd, fx);
+  fy = nmad(vy, rd, fy);
+  fz = nmad(vz, rd, fz);
+  const R q = d_div(dot3(fx, bx, fy, by, fz, bz), d_fmax(tiny100<R>(), bb));
+  const R b0 = -bf * nmad(q, bx, fx), b1 = -bf * nmad(q, by, fy), b2 = -bf * nmad(q, bz, fz);
+  const R b3 = dot3(b0, vx, b1, vy, b2, vz);
   Racc[1] += b0;
   Racc[2] += b1;
   Racc[3] += b2;
@@ -732,15 +731,15 @@ __device__ __forceinline__ void tvd_cell(const Consts& c, const Raw9<R>& r, R hb
   v1 = v1 * dn;
   v2 = v2 * dn;
   v3 = v3 * dn;
-  R vv = v1 * v1 + v2 * v2 + v3 * v3;
-  R bb = b5 * b5 + b6 * b6 + b7 * b7;
-  e = e * dn - d_half(vv);
+  R vv = dot3(v1, v1, v2, v2, v3, v3);
+  R bb = dot3(b5, b5, b6, b6, b7, b7);
+  e = mad(e, dn, -d_half(vv));
   t.vsqr = vv;
   t.bsqr = bb;
   vv = d_sqrt(vv);
   R va2 = bb * dn;
-  R x2 = va2 * inv_va2max, x4 = x2 * x2, s = (R)1.0 + x2;
-  R lf = d_div(s, s + x4);
+  R x2 = va2 * inv_va2max, s = (R)1.0 + x2;
+  R lf = d_div(s, mad(x2, x2, s));
   R cs2 = (R)(5.0 / 3.0) * r.v[8] * dn;
   const R CZ = k.CZ;
   // FP64: with CZ = 1 (full optical depth) the Mach-number damping CME is zero
@@ -759,11 +758,11 @@ __device__ __forceinline__ void tvd_cell(const Consts& c, const Raw9<R>& r, R hb
   // vertical boundaries; there their terms add nothing and hh is 1
   if (std::is_same<R, double>::value && t.hb == (R)0.0 && t.ht == (R)0.0) {
     const R ro = (R)1.0 - rf;
-    cf = rf * k.tvd_cs[1] + ro * k.tvd_cs[2];
+    cf = mad(rf, k.tvd_cs[1], ro * k.tvd_cs[2]);
     const R a1 = rf * h1, a2 = ro * h2;
     t.he = a1 + a2;
-    t.hv = a1 + a2 * k.pm_v;
-    t.hB = a1 + a2 * k.pm_B;
+    t.hv = mad(a2, k.pm_v, a1);
+    t.hB = mad(a2, k.pm_B, a1);
   } else {
     cf = t.hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + ((R)1.0 - rf) * k.tvd_cs[2]) * hh + t.ht * k.tvd_cs[3];
     t.he = t.hb * h0 + (rf * h1 + ((R)1.0 - rf) * h2) * hh + t.ht * h3;
@@ -844,7 +843,7 @@ __device__ __forceinline__ void tvd_flux(const Consts& c, const TCell<R>& am, co
     R dn = (v >= 1 && v <= 3) ? a.hv : ((v >= 5) ? a.hB : a.he);
     R rf = d_div(d_fabs(sl_lim), smax(tiny100<R>(), d_fabs(sl)));
     R cf = smax((R)0.0, smin(sl_lim, sl)) + smin((R)0.0, smax(sl_lim, sl));
-    F[v] = smax((R)0.0, (R)1.0 + dn * (rf - (R)1.0)) * cf;
+    F[v] = smax((R)0.0, mad(dn, rf - (R)1.0, (R)1.0)) * cf;
   }
   R fac = fac0 * smin(cmax_t, smax(a.cm, b.cm));
 #pragma unroll
@@ -877,18 +876,19 @@ __device__ __forceinline__ void tvd_flux(const Consts& c, const TCell<R>& am, co
   }
   const R CZ = k.CZ;
   R min_cz = f0 * smin(CZ, CZ);
-  f1 *= u[0]; f1 += u[1] * min_cz;
-  f2 *= u[0]; f2 += u[2] * min_cz;
-  f3 *= u[0]; f3 += u[3] * min_cz;
+  f1 = mad(u[1], min_cz, f1 * u[0]);
+  f2 = mad(u[2], min_cz, f2 * u[0]);
+  f3 = mad(u[3], min_cz, f3 * u[0]);
   f4 *= u[0];
-  if (std::is_same<R, double>::value && a.qt == (R)1.0) f4 += (u[4] * min_cz) + (u[1] * f1 + u[2] * f2 + u[3] * f3);
-  else f4 += (u[4] * min_cz) + a.qt * (u[1] * f1 + u[2] * f2 + u[3] * f3);
+  const R uf = dot3(u[1], f1, u[2], f2, u[3], f3);
+  if (std::is_same<R, double>::value && a.qt == (R)1.0) f4 += mad(u[4], min_cz, uf);
+  else f4 += (u[4] * min_cz) + a.qt * uf;
   F[0] = f0; F[1] = f1; F[2] = f2; F[3] = f3; F[4] = f4;
   if (DIR == 0 && !c.g.periodic_x) {
     if (ia == sz - GH - 1) F[5] = (R)0.0;
     if (ia == GH - 1) F[5] = (R)0.0;
   }
-  qres = (b.q[5] - a.q[5]) * F[5] + (b.q[6] - a.q[6]) * F[6] + (b.q[7] - a.q[7]) * F[7];
+  qres = dot3(b.q[5] - a.q[5], F[5], b.q[6] - a.q[6], F[6], b.q[7] - a.q[7], F[7]);
   // viscous heating at the interface, for the diagnostics (src/tvdlimit_SR.C:626-635)
   if (DIAG) *qvis = (b.q[1] - a.q[1]) * F[1] + (b.q[2] - a.q[2]) * F[2] + (b.q[3] - a.q[3]) * F[3];
 }
@@ -919,17 +919,17 @@ __device__ __forceinline__ void tvd_update(const Consts& c, R dtt, const R* Fp, 
     res[4] += ((R)1.0 - c0.qt) * (res[1] * c0.q[1] + res[2] * c0.q[2] + res[3] * c0.q[3]);
   if (DIAG) dg->d[7 * N + id] += res[4] * dg->idt_full;
   {
-    R dn = d_div(res[1] * c0.q[5] + res[2] * c0.q[6] + res[3] * c0.q[7], smax(tiny100<R>(), c0.bsqr));
-    R b0 = -c0.BC2 * (res[1] - dn * c0.q[5]);
-    R b1 = -c0.BC2 * (res[2] - dn * c0.q[6]);
-    R b2 = -c0.BC2 * (res[3] - dn * c0.q[7]);
-    R b3 = b0 * c0.q[1] + b1 * c0.q[2] + b2 * c0.q[3];
+    R dn = d_div(dot3(res[1], c0.q[5], res[2], c0.q[6], res[3], c0.q[7]), smax(tiny100<R>(), c0.bsqr));
+    R b0 = -c0.BC2 * nmad(dn, c0.q[5], res[1]);
+    R b1 = -c0.BC2 * nmad(dn, c0.q[6], res[2]);
+    R b2 = -c0.BC2 * nmad(dn, c0.q[7], res[3]);
+    R b3 = dot3(b0, c0.q[1], b1, c0.q[2], b2, c0.q[3]);
     res[1] += b0; res[2] += b1; res[3] += b2; res[4] += b3;
     if (DIAG) dg->d[5 * N + id] += b3 * dg->idt_full;
   }
   {
     R qres = d_half(qp + qm) * c0.qt;
-    res[4] += dtt * qres;
+    res[4] = mad(dtt, qres, res[4]);
     if (DIAG) dg->d[8 * N + id] += dg->dt_fac * qres;
   }
   if constexpr (std::is_same<R, float>::value) {
@@ -958,7 +958,7 @@ __device__ __forceinline__ void tvd_update(const Consts& c, R dtt, const R* Fp, 
   for (int v = 0; v < NV; v++) u[v] = u_in[v] + res[v];
   u[0] = smax((R)kk_.rho_min, u[0]);
   const R eb = u[4];
-  u[4] = smax(u[4], kk_.eps_min * u[0] + d_div(d_half(u[1] * u[1] + u[2] * u[2] + u[3] * u[3]), u[0]));
+  u[4] = smax(u[4], mad(kk_.eps_min, u[0], d_div(d_half(dot3(u[1], u[1], u[2], u[2], u[3], u[3])), u[0])));
   if (DIAG) {
     dg->d[6 * N + id] += (u[4] - eb) * dg->idt_full;
     dg->d[9 * N + id] += dg->dt_fac * ((R)0.5 * (qvp + qvm) * c0.qt);

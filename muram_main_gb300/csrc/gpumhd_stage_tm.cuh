@@ -210,7 +210,7 @@ __device__ __forceinline__ void tm_deriv12(double* Dq, unsigned m2, unsigned m1,
         return __longlong_as_double((long long)(((unsigned long long)r[o + 1] << 32) | (unsigned long long)r[o]));
       };
       const double a2 = dbl(2 * h), a1 = dbl(4 + 2 * h), b1 = dbl(8 + 2 * h), b2 = dbl(12 + 2 * h);
-      Dq[2 * a + h] = w1 * (b1 - a1) + w2 * (b2 - a2);
+      Dq[2 * a + h] = mad(w1, b1 - a1, w2 * (b2 - a2));
     }
   }
 }

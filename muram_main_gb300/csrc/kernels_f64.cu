@@ -1,5 +1,5 @@
-// FP64 kernels: compiled with --fmad=false so that every product and sum
-// rounds separately, as in the reference's no-FMA builds.
+// FP64 kernels: compiled with --fmad=false, so that fused multiply-adds are
+// those the sources write (mad) and no others.
 #define GPUMHD_LAUNCH_IMPL
 #include "gpumhd_launch.cuh"
 

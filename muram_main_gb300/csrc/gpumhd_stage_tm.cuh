@@ -103,12 +103,12 @@ __device__ __forceinline__ void tmem_ld4(unsigned t, unsigned& a, unsigned& b, u
                : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Waits for this thread's tensor-memory loads; the 16 registers pass through
+// Waits for this thread's tensor-memory loads; the 12 registers pass through
 // the instruction so that no use of them is scheduled before it.
-__device__ __forceinline__ void tmem_wait_ld16(unsigned* r) {
+__device__ __forceinline__ void tmem_wait_ld12(unsigned* r) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11])
                :
                : "memory");
 }
@@ -127,12 +127,9 @@ struct StageTm {
   // one barrier per plane suffices (the next plane's fluxes go to the other
   // buffer; a slot is refilled right after the barrier of the plane that
   // last reads it).  Otherwise four slots and one flux buffer, two barriers
-  // per plane.  Two blocks per SM fit either way in FP32; FP64 uses the
-  // latter only.  Measured at 128 x 384 x 384 (FP32): DB is faster for the
-  // stages that read no separate U0 (stage 1: 0.76 against 0.79 ms; stage 4,
-  // whose U0 is its output, 0.62 against 0.67 ms; the residual), slower for
-  // stages 2 and 3 (0.80 against 0.78 ms), whose U0 loads and EOS gathers
-  // then have less L1 beside the larger shared memory.
+  // per plane.  Two blocks per SM fit either way in FP32; FP64 uses the latter
+  // only.  Measured at 128 x 384 x 384 (FP32): DB 645 against 670 us in stage 1,
+  // 674 against 680 in stages 2 and 3, 554 against 568 in stage 4.
   static constexpr bool DB = DB_;
   static constexpr int NSLOT = DB ? 3 : 4;
   static constexpr int NFB = DB ? 2 : 1;
@@ -167,25 +164,25 @@ __device__ __forceinline__ void tm_store12(unsigned ta, const double* f) {
   }
 }
 
-// z derivative of the 12 quantities from the ring slots of planes k-2, k-1,
-// k+1, k+2 (column addresses m2, m1, p1, p2), in the order of deriv12.
-__device__ __forceinline__ void tm_deriv12(float* Dq, unsigned m2, unsigned m1, unsigned p1, unsigned p2, float w1,
+// z derivative of the 12 quantities from the ring slots of planes k-2, k-1, k+1
+// (column addresses m2, m1, p1) and the fluxes f2 of plane k+2, in the order of
+// deriv12.
+__device__ __forceinline__ void tm_deriv12(float* Dq, unsigned m2, unsigned m1, unsigned p1, const float* f2, float w1,
                                            float w2) {
   const float2 neg = make_float2(-1.0f, -1.0f), W1 = make_float2(w1, w1), W2 = make_float2(w2, w2);
 #pragma unroll
   for (int a = 0; a < 3; a++) {
-    unsigned r[16];
+    unsigned r[12];
     tm::tmem_ld4(m2 + 4 * a, r[0], r[1], r[2], r[3]);
     tm::tmem_ld4(m1 + 4 * a, r[4], r[5], r[6], r[7]);
     tm::tmem_ld4(p1 + 4 * a, r[8], r[9], r[10], r[11]);
-    tm::tmem_ld4(p2 + 4 * a, r[12], r[13], r[14], r[15]);
-    tm::tmem_wait_ld16(r);
+    tm::tmem_wait_ld12(r);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const float2 a2 = make_float2(__uint_as_float(r[2 * h]), __uint_as_float(r[2 * h + 1]));
       const float2 a1 = make_float2(__uint_as_float(r[4 + 2 * h]), __uint_as_float(r[5 + 2 * h]));
       const float2 b1 = make_float2(__uint_as_float(r[8 + 2 * h]), __uint_as_float(r[9 + 2 * h]));
-      const float2 b2 = make_float2(__uint_as_float(r[12 + 2 * h]), __uint_as_float(r[13 + 2 * h]));
+      const float2 b2 = make_float2(f2[4 * a + 2 * h], f2[4 * a + 2 * h + 1]);
       const float2 d1 = __ffma2_rn(a1, neg, b1);
       const float2 d2 = __ffma2_rn(a2, neg, b2);
       const float2 res = __ffma2_rn(W1, d1, __fmul2_rn(W2, d2));
@@ -194,22 +191,21 @@ __device__ __forceinline__ void tm_deriv12(float* Dq, unsigned m2, unsigned m1, 
     }
   }
 }
-__device__ __forceinline__ void tm_deriv12(double* Dq, unsigned m2, unsigned m1, unsigned p1, unsigned p2, double w1,
+__device__ __forceinline__ void tm_deriv12(double* Dq, unsigned m2, unsigned m1, unsigned p1, const double* f2, double w1,
                                            double w2) {
 #pragma unroll
   for (int a = 0; a < 6; a++) {
-    unsigned r[16];
+    unsigned r[12];
     tm::tmem_ld4(m2 + 4 * a, r[0], r[1], r[2], r[3]);
     tm::tmem_ld4(m1 + 4 * a, r[4], r[5], r[6], r[7]);
     tm::tmem_ld4(p1 + 4 * a, r[8], r[9], r[10], r[11]);
-    tm::tmem_ld4(p2 + 4 * a, r[12], r[13], r[14], r[15]);
-    tm::tmem_wait_ld16(r);
+    tm::tmem_wait_ld12(r);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       auto dbl = [&](int o) {
         return __longlong_as_double((long long)(((unsigned long long)r[o + 1] << 32) | (unsigned long long)r[o]));
       };
-      const double a2 = dbl(2 * h), a1 = dbl(4 + 2 * h), b1 = dbl(8 + 2 * h), b2 = dbl(12 + 2 * h);
+      const double a2 = dbl(2 * h), a1 = dbl(4 + 2 * h), b1 = dbl(8 + 2 * h), b2 = f2[2 * a + h];
       Dq[2 * a + h] = mad(w1, b1 - a1, w2 * (b2 - a2));
     }
   }
@@ -373,16 +369,6 @@ __global__ void __launch_bounds__(TX* TY, 2)
     if (!L::DB && tid == 0 && k + 1 < ze) issue(k + 3);
     R* const FX = fx_of(L::DB ? ((k - zb) & 1) : 0);
     R* const FY = FX + 12 * L::FXN;
-    // z flux of plane k+2 (all lanes: tensor-memory stores are warp-wide)
-    wait_slot(sl_n, ph_n);
-    __syncwarp();
-    {
-      Raw9<R> r;
-      raw_at(tile_at(sl_n), o_own, r);
-      prim_of_raw<R, RESID>(r, prim);
-      flux12<R, 2>(prim, 1, fl, 1);
-      tm_store12(zcol(slot_add(s0, 2)), fl);
-    }
     // own cell: primitives and x / y fluxes; halo cell: its x or y flux
     R cen[NF];
     {
@@ -420,16 +406,25 @@ __global__ void __launch_bounds__(TX* TY, 2)
       }
     }
     if (pend) finish_pressure(k - 1);
-    tm::tmem_wait_st();
+    tm::tmem_wait_st();  // the previous plane's z flux
     __syncthreads();
     // FP32: plane k's slot is free (its last reads were this plane's own and
     // halo cells), refill it with plane k+3, read in the next plane
     if (L::DB && tid == 0 && k + 1 < ze) issue(k + 3);
-    // z derivative (all lanes), then the cell's residual and update
+    // z flux of plane k+2 (all lanes: tensor-memory accesses are warp-wide), kept
+    // in registers for this plane's derivative and stored for the next ones
+    // (stored before the barrier and loaded back it took 25 us more per stage)
     R Dz[NF];
+    wait_slot(sl_n, ph_n);
     __syncwarp();
-    tm_deriv12(Dz, zcol(slot_add(s0, 3)), zcol(slot_add(s0, 4)), zcol(slot_add(s0, 1)), zcol(slot_add(s0, 2)),
-               kk_.w1[2], kk_.w2[2]);
+    {
+      Raw9<R> r;
+      raw_at(tile_at(sl_n), o_own, r);
+      prim_of_raw<R, RESID>(r, prim);
+      flux12<R, 2>(prim, 1, fl, 1);
+      tm_deriv12(Dz, zcol(slot_add(s0, 3)), zcol(slot_add(s0, 4)), zcol(slot_add(s0, 1)), fl, kk_.w1[2], kk_.w2[2]);
+      tm_store12(zcol(slot_add(s0, 2)), fl);
+    }
     if (active) {
       R Racc[NV];  // fused stage: written by the first direction
       if (RESID) {

@@ -406,7 +406,7 @@ def run_ours(args):
                 "design_bytes_per_launch": design_bytes_per_launch,
                 "peak_source": f"{peak_src} hbm_gbs"}
     if dom == "stage":
-        roofline["limiter"] = ("instruction issue and dependency latency, not HBM (ncu: ~58 % issue active, "
+        roofline["limiter"] = ("instruction issue and dependency latency, not HBM (ncu: ~50 % issue active, "
                                "24-39 % DRAM throughput)")
     # whole-step bytes against HBM
     step_bytes = ALGO_STEP_WORDS * 4 * n_cells
@@ -498,11 +498,6 @@ def run_ours(args):
                 "roofline": {"bound": "fp64", "kernel": "k_stage_tm (FP64, RK stages 1-4)",
                              "achieved": round(ach64, 4), "peak": round(peak64, 4), "unit": "TFLOP/s",
                              "frac": round(ach64 / peak64, 4), "mean_launch_ms": round(stage64_ms, 4),
-                             # the FP64 mode is compiled without FMA contraction (parity with the
-                             # reference's no-FMA build): one flop per FP64 instruction, half the
-                             # DGEMM's flops per instruction
-                             "peak_without_fma": round(peak64 / 2, 4),
-                             "frac_without_fma": round(ach64 / (peak64 / 2), 4),
                              "flops_per_cell_per_launch": FLOPS_STAGE_PER_CELL,
                              "peak_source": "measured: cuBLAS DGEMM 8192^3 via torch.matmul",
                              "hbm_frac": round(ALGO_STAGE_WORDS / 4 * 8 * n_cells / (stage64_ms / 1e3) / 1e9

@@ -96,14 +96,14 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
   const double F[3] = {R[1] + dn2, R[2], R[3]};
   const double rd = R[0];
   const double bb = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
-  const double va2 = bb / rh;
+  const double va2 = d_div(bb, rh);
   const double x2 = va2 * inv_va2max, x4 = x2 * x2;
   const double D = 1.0 + x2 + x4;
-  const double bf = x4 / D;
+  const double bf = d_div(x4, D);
   double f[3], bo[3];
   for (int i = 0; i < 3; i++) f[i] = F[i] - v[i] * rd;
   const double bq = d_fmax(tiny, bb);
-  const double q = (f[0] * B[0] + f[1] * B[1] + f[2] * B[2]) / bq;
+  const double q = d_div(f[0] * B[0] + f[1] * B[1] + f[2] * B[2], bq);
   for (int i = 0; i < 3; i++) bo[i] = -bf * (f[i] - q * B[i]);
   // ---- reverse
   double l_v[3] = {0.0, 0.0, 0.0}, l_B[3] = {0.0, 0.0, 0.0}, l_f[3];
@@ -116,8 +116,8 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
     l_q += bf * l_bo * B[i];
     l_B[i] += bf * l_bo * q;
   }
-  const double l_Nq = l_q / bq;  // q = (f . B) / max(tiny, bb)
-  double l_bb = (tiny < bb) ? -l_q * q / bq : 0.0;
+  const double l_Nq = d_div(l_q, bq);  // q = (f . B) / max(tiny, bb)
+  double l_bb = (tiny < bb) ? d_div(-l_q * q, bq) : 0.0;
   for (int i = 0; i < 3; i++) {
     l_f[i] += l_Nq * B[i];
     l_B[i] += l_Nq * f[i];
@@ -128,12 +128,12 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
     l_v[i] -= l_f[i] * rd;
     l_rd -= l_f[i] * v[i];
   }
-  const double l_D = -l_bf * bf / D;  // bf = x4 / ((1 + x2) + x4)
-  const double l_x4 = l_bf / D + l_D;
+  const double l_D = d_div(-l_bf * bf, D);  // bf = x4 / ((1 + x2) + x4)
+  const double l_x4 = d_div(l_bf, D) + l_D;
   const double l_x2 = l_D + l_x4 * 2.0 * x2;
   const double l_va2 = l_x2 * inv_va2max;
-  l_bb += l_va2 / rh;
-  double l_rh = -l_va2 * va2 / rh;
+  l_bb += d_div(l_va2, rh);
+  double l_rh = d_div(-l_va2 * va2, rh);
   for (int i = 0; i < 3; i++) l_B[i] += l_bb * 2.0 * B[i];
   const double l_R1 = lG[1] + l_F[0];  // R[1] + dn2 is both the output and fx
   l_R[0] = lG[0] + l_rd;
@@ -154,14 +154,14 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
 // Reverse of boris_lf<double> (src/mhdres_SR.C:310-323): l_lf back to the
 // cell's density and field (l_cen, added).
 __device__ __forceinline__ void boris_lf_rev(const double* cen, double inv_va2max, double l_lf, double* l_cen) {
-  const double dn = 1.0 / cen[P_D];
+  const double dn = d_div(1.0, cen[P_D]);
   const double B[3] = {cen[P_B1], cen[P_B2], cen[P_B3]};
   const double bb = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
   const double va2 = bb * dn;
   const double x2 = va2 * inv_va2max, x4 = x2 * x2, s = 1.0 + x2;
-  const double E = s + x4, lf = s / E;
-  const double l_s = l_lf * (1.0 - lf) / E;  // lf = s / (s + x4)
-  const double l_x4 = -l_lf * lf / E;
+  const double E = s + x4, lf = d_div(s, E);
+  const double l_s = d_div(l_lf * (1.0 - lf), E);  // lf = s / (s + x4)
+  const double l_x4 = d_div(-l_lf * lf, E);
   const double l_x2 = l_s + l_x4 * 2.0 * x2;
   const double l_va2 = l_x2 * inv_va2max;
   const double l_bb = l_va2 * dn, l_dn = l_va2 * bb;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void flux12_rev(const double* p, const double* lF, do
 // residual's kinetic and magnetic pressures): lw, the adjoints of the 11
 // primitives, back to the cell's 9 stored values (lr, written).
 __device__ __forceinline__ void prim_of_raw_rev(const Raw9<double>& r, const double* lw, double* lr) {
-  const double d = r.v[0], dn = 1.0 / d;
+  const double d = r.v[0], dn = d_div(1.0, d);
   const double m[3] = {r.v[1], r.v[2], r.v[3]};
   double v[3];
   for (int t = 0; t < 3; t++) v[t] = m[t] * dn;
@@ -495,7 +495,7 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
     sll[v] = b.q[v] - a.q[v] - (sa[v] + sb[v]);
     const double dnv = tf(a)[dn_field(v)];
     den[v] = smax(tiny, fabs(sl[v]));
-    rf[v] = fabs(sll[v]) / den[v];
+    rf[v] = d_div(fabs(sll[v]), den[v]);
     cfv[v] = smax(0.0, smin(sll[v], sl[v])) + smin(0.0, smax(sll[v], sl[v]));
     G[v] = smax(0.0, 1.0 + dnv * (rf[v] - 1.0));
     F0[v] = G[v] * cfv[v];
@@ -535,9 +535,9 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
   for (int v = 0; v < 5; v++) u[v] = 0.5 * (a.q[v] + sa[v] + b.q[v] - sb[v]);
   double U0 = u[0], U4 = u[4], f0 = F[0], f4a = F[4];
   if (c.rho_log) {
-    U0 = exp(u[0]);
+    U0 = d_exp(u[0]);
     f0 = F[0] * U0;
-    U4 = exp(u[4]);
+    U4 = d_exp(u[4]);
     f4a = F[4] * U4;
   }
   const double CZ = smin(k.CZ, k.CZ);
@@ -645,8 +645,8 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
       l_rf = l_G * dnv;
     }
     double l_sl = 0.0, l_sll = 0.0;
-    l_sll += (l_rf / den[v]) * (sll[v] < 0.0 ? -1.0 : 1.0);  // rf = |sll| / den
-    if (tiny < fabs(sl[v])) l_sl += (-l_rf * rf[v] / den[v]) * (sl[v] < 0.0 ? -1.0 : 1.0);
+    l_sll += d_div(l_rf, den[v]) * (sll[v] < 0.0 ? -1.0 : 1.0);  // rf = |sll| / den
+    if (tiny < fabs(sl[v])) l_sl += d_div(-l_rf * rf[v], den[v]) * (sl[v] < 0.0 ? -1.0 : 1.0);
     if (0.0 < smin(sll[v], sl[v])) {  // cf = max(0, min(sll, sl)) + min(0, max(sll, sl))
       if (sl[v] < sll[v]) l_sl += l_cf;
       else l_sll += l_cf;
@@ -680,7 +680,7 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
   const double r4a = res[4] + (1.0 - c0.qt) * W;
   const double bs = smax(tiny, c0.bsqr);
   const double num = res[1] * c0.q[5] + res[2] * c0.q[6] + res[3] * c0.q[7];
-  const double dn = num / bs;
+  const double dn = d_div(num, bs);
   double bb[3];
   for (int t = 0; t < 3; t++) bb[t] = -c0.BC2 * (res[1 + t] - dn * c0.q[5 + t]);
   const double b3 = bb[0] * c0.q[1] + bb[1] * c0.q[2] + bb[2] * c0.q[3];
@@ -695,7 +695,7 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
   for (int v = 0; v < NV; v++) u[v] = u_in[v] + r[v];
   const double u0f = smax(k.rho_min, u[0]);
   const double K = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
-  const double ef = k.eps_min * u0f + 0.5 * K / u0f;
+  const double ef = k.eps_min * u0f + d_div(0.5 * K, u0f);
   // ---- reverse
   double l_u[NV];
 #pragma unroll
@@ -705,8 +705,8 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
     l_ef = lu[4];
     l_u[4] = 0.0;
   }
-  double l_u0f = lu[0] + l_ef * (k.eps_min - 0.5 * K / (u0f * u0f));
-  for (int t = 1; t <= 3; t++) l_u[t] += l_ef * u[t] / u0f;
+  double l_u0f = lu[0] + l_ef * (k.eps_min - d_div(0.5 * K, u0f * u0f));
+  for (int t = 1; t <= 3; t++) l_u[t] += d_div(l_ef * u[t], u0f);
   l_u[0] = (k.rho_min < u[0]) ? l_u0f : 0.0;  // u0 = max(rho_min, u0)
 #pragma unroll
   for (int v = 0; v < NV; v++) l_in[v] = l_u[v];
@@ -733,8 +733,8 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
     l_dn -= l_inn * c0.q[5 + t];
     l_c0[5 + t] -= l_inn * dn;
   }
-  const double l_num = l_dn / bs;  // dn = num / bs
-  if (tiny < c0.bsqr) l_c0[T_BSQR] += -l_dn * dn / bs;
+  const double l_num = d_div(l_dn, bs);  // dn = num / bs
+  if (tiny < c0.bsqr) l_c0[T_BSQR] += d_div(-l_dn * dn, bs);
   for (int t = 0; t < 3; t++) {
     l_res[1 + t] += l_num * c0.q[5 + t];
     l_c0[5 + t] += l_num * res[1 + t];
@@ -766,7 +766,7 @@ __device__ void tvd_slope_rev(const Consts& c, const TCell<double>& a, const TCe
   double ls[NV];
 #pragma unroll
   for (int v = 0; v < NV; v++) ls[v] = ls_in[v];
-  const double qr = c.rho_log ? fabs(b.q[0] - n.q[0]) : fabs(log(b.q[0]) - log(n.q[0]));
+  const double qr = c.rho_log ? fabs(b.q[0] - n.q[0]) : fabs(d_log(b.q[0]) - d_log(n.q[0]));
   if (qr > k.q_rho_max) ls[0] = 0.0;
   if (k.has_vmax_lim && b.vsqr > vsqr_diff) ls[1] = ls[2] = ls[3] = 0.0;
   double s0[NV];  // the limited slopes before the boundary factors
@@ -829,21 +829,21 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
   // ---- forward
   const double d0 = r.v[0];
   const double d = smax(k.rho_min, d0);
-  const double dn = 1.0 / d;
+  const double dn = d_div(1.0, d);
   double v[3], Bc[3];
   for (int t = 0; t < 3; t++) { v[t] = r.v[1 + t] * dn; Bc[t] = r.v[5 + t]; }
   const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const double bb = Bc[0] * Bc[0] + Bc[1] * Bc[1] + Bc[2] * Bc[2];
   const double e = r.v[4] * dn - 0.5 * vv;
-  const double vs = sqrt(vv);
+  const double vs = d_sqrt(vv);
   const double va2 = bb * dn;
   const double x2 = va2 * inv_va2max, x4 = x2 * x2, s = 1.0 + x2, E = s + x4;
-  const double lf = s / E;
+  const double lf = d_div(s, E);
   const double cs2 = (5.0 / 3.0) * r.v[8] * dn;
-  const double cfast = sqrt(va2 + cs2);
+  const double cfast = d_sqrt(va2 + cs2);
   const double CME = (1.0 - k.CZ) * ((double)(vs >= k.CME_thresh * cfast));
   const double d2 = d * d;
-  const double rl = d2 / (d2 + k.rho_lev);
+  const double rl = d_div(d2, d2 + k.rho_lev);
   const double rf = smin(lf, rl);
   const double hh = 1.0 - hb - ht;
   const double cfa = hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + (1.0 - rf) * k.tvd_cs[2]) * hh + ht * k.tvd_cs[3];
@@ -851,11 +851,11 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
   const double cs2b = cs2 * (cf * cf);
   const double A = lf * (cs2b + va2);
   const double mx = smax(cs2b, A);
-  const double sq = sqrt(mx);
+  const double sq = d_sqrt(mx);
   const double cm = 0.0 + vs + sq;
   // ---- reverse
-  double l_d = c.rho_log ? lt[0] / d : lt[0];
-  const double l_e = c.rho_log ? lt[4] / e : lt[4];
+  double l_d = c.rho_log ? d_div(lt[0], d) : lt[0];
+  const double l_e = c.rho_log ? d_div(lt[4], e) : lt[4];
   double l_v[3], l_B[3];
   for (int t = 0; t < 3; t++) { l_v[t] = lt[1 + t]; l_B[t] = lt[5 + t]; }
   double l_cm = lt[T_CM], l_vv = lt[T_VSQR], l_bb = lt[T_BSQR], l_lf = -lt[T_BC2];
@@ -865,14 +865,14 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
     if (0.0 < mn) {
       const double l_mn = lt[T_HD] * fac0;
       if (g < hv) l_cm -= l_mn;
-      else if (vs > 0.0) l_vv += l_mn * k.vhyp * 0.5 / vs;
+      else if (vs > 0.0) l_vv += d_div(l_mn * k.vhyp * 0.5, vs);
     }
   }
   const double h1 = k.tvd_h[1], h2 = k.tvd_h[2];
   double l_rf = (lt[T_HE] * (1.0 - CME) * (h1 - h2) + lt[T_HV] * (1.0 - CME) * (h1 - h2 * k.pm_v) +
                  lt[T_HB] * (h1 - h2 * k.pm_B)) * hh;
   double l_vs = l_cm;  // cm = (0 + vs) + sqrt(mx)
-  const double l_mx = sq > 0.0 ? l_cm * 0.5 / sq : 0.0;
+  const double l_mx = sq > 0.0 ? d_div(l_cm * 0.5, sq) : 0.0;
   double l_cs2b = 0.0, l_A = 0.0;
   if (cs2b < A) l_A = l_mx;
   else l_cs2b = l_mx;
@@ -882,15 +882,15 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
   double l_cs2 = l_cs2b * (cf * cf);
   const double l_cf = l_cs2b * cs2 * 2.0 * cf;
   if (!(cfa < CME)) l_rf += l_cf * (k.tvd_cs[1] - k.tvd_cs[2]) * hh;
-  if (rl < lf) l_d += l_rf * k.rho_lev / ((d2 + k.rho_lev) * (d2 + k.rho_lev)) * 2.0 * d;
+  if (rl < lf) l_d += d_div(l_rf * k.rho_lev, (d2 + k.rho_lev) * (d2 + k.rho_lev)) * 2.0 * d;
   else l_lf += l_rf;
   double l_dn = l_cs2 * (5.0 / 3.0) * r.v[8];
   lr[8] = l_cs2 * (5.0 / 3.0) * dn;
-  const double l_x2 = l_lf * (1.0 - lf) / E + (-l_lf * lf / E) * 2.0 * x2;  // lf = s / (s + x4)
+  const double l_x2 = d_div(l_lf * (1.0 - lf), E) + d_div(-l_lf * lf, E) * 2.0 * x2;  // lf = s / (s + x4)
   l_va2 += l_x2 * inv_va2max;
   l_bb += l_va2 * dn;  // va2 = bb * dn
   l_dn += l_va2 * bb;
-  if (vs > 0.0) l_vv += l_vs * 0.5 / vs;
+  if (vs > 0.0) l_vv += d_div(l_vs * 0.5, vs);
   lr[4] = l_e * dn;  // e = r4 * dn - 0.5 * vv
   l_dn += l_e * r.v[4];
   l_vv -= 0.5 * l_e;

@@ -52,7 +52,7 @@ template <int K> __device__ __forceinline__ double val(const Dual<K>& x) { retur
 GPUMHD_DUAL_BINOP(+, a.v + b.v, a.d[k] + b.d[k])
 GPUMHD_DUAL_BINOP(-, a.v - b.v, a.d[k] - b.d[k])
 GPUMHD_DUAL_BINOP(*, a.v * b.v, a.d[k] * b.v + a.v * b.d[k])
-GPUMHD_DUAL_BINOP(/, a.v / b.v, (a.d[k] * b.v - a.v * b.d[k]) / (b.v * b.v))
+GPUMHD_DUAL_BINOP(/, d_div(a.v, b.v), d_div(a.d[k] * b.v - a.v * b.d[k], b.v * b.v))
 #undef GPUMHD_DUAL_BINOP
 
 template <int K> __device__ __forceinline__ Dual<K> operator-(const Dual<K>& a) {
@@ -90,12 +90,12 @@ template <int K> __device__ __forceinline__ Dual<K> dual_chain(const Dual<K>& a,
   return r;
 }
 template <int K> __device__ __forceinline__ Dual<K> d_sqrt(const Dual<K>& a) {
-  const double s = sqrt(a.v);
-  return dual_chain(a, s, s > 0.0 ? 0.5 / s : 0.0);
+  const double s = d_sqrt(a.v);
+  return dual_chain(a, s, s > 0.0 ? d_div(0.5, s) : 0.0);
 }
-template <int K> __device__ __forceinline__ Dual<K> d_log(const Dual<K>& a) { return dual_chain(a, log(a.v), 1.0 / a.v); }
+template <int K> __device__ __forceinline__ Dual<K> d_log(const Dual<K>& a) { return dual_chain(a, d_log(a.v), d_div(1.0, a.v)); }
 template <int K> __device__ __forceinline__ Dual<K> d_exp(const Dual<K>& a) {
-  const double e = exp(a.v);
+  const double e = d_exp(a.v);
   return dual_chain(a, e, e);
 }
 template <int K> __device__ __forceinline__ Dual<K> d_fabs(const Dual<K>& a) {

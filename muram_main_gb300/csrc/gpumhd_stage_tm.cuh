@@ -521,6 +521,10 @@ __global__ void __launch_bounds__(TX* TY, 2)
 
   // teardown: report an expired wait, let issued copies land, free tensor memory
   if (timed_out) atomicExch(&misc[2], 1u);
+  // the last plane's stores: another block may be given these columns as soon as
+  // they are freed
+  __syncwarp();
+  tm::tmem_wait_st();
   tm::tc_fence_before();
   __syncthreads();
   if (misc[2]) {

@@ -81,7 +81,7 @@ struct gpumhd_ctx {
   // test hook of the TMA stage kernel's bounded waits (gpumhd_test_tma_wait)
   int tm_withhold_last = 0;
   long long tm_wait_cycles = 0;
-  void* comp = nullptr;  // FP32 compensated mode: per-cell remainders of the RK update (8N floats)
+  void* comp = nullptr;  // FP32 compensated mode: per-cell rounding remainders (8N), then the x sweep's (8N)
   // diagnostics of an output step (RunData::need_diagnostics): tvar1..tvar8,
   // Qres, Qvis (GridData, 10 x N), allocated when first switched on
   void* diag = nullptr;
@@ -1647,7 +1647,7 @@ static int fused_prepare(gpumhd_ctx* ctx, int nsteps) {
     if (rc1) return rc1;
   }
   if (ctx->f32 && ctx->p.compensated && !ctx->comp) {
-    CK(cudaMalloc(&ctx->comp, sizeof(Rem<float>) * 8 * ctx->c.g.N));
+    CK(cudaMalloc(&ctx->comp, sizeof(Rem<float>) * 16 * ctx->c.g.N));
     CK(cudaMemsetAsync(ctx->comp, 0, sizeof(Rem<float>) * 8 * ctx->c.g.N, ctx->stream));
   }
   if (!ctx->fused_ready) {

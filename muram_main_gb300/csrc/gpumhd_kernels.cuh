@@ -1106,11 +1106,15 @@ __global__ void __launch_bounds__(FIN_BX* FIN_BY, FinBlocks<R>::v) k_step_finish
 // few spilled), the x sweep 0.623 -> 0.603 ms with 6 (85 registers).
 template <class R> struct TvdBlocks { static constexpr int pencil = sizeof(R) == 4 ? 4 : 1, lanes = sizeof(R) == 4 ? 6 : 1; };
 
-// COMP: FP32 compensated fused steps (Cc: the state's rounding remainders).
+// COMP: FP32 compensated fused steps; Ci, Co: the state's rounding remainders
+// before and after the sweep.  A ghost row reads the remainder of the interior
+// cell it images, which that cell's own thread replaces, so the sweeps with
+// ghost rows read one array and write another: x Cc -> second array, y back; z,
+// without ghost rows, in place.
 template <class R, int DIR, bool DIAG = false, bool COMP = false>
 __global__ void __launch_bounds__(128, TvdBlocks<R>::pencil) k_tvd_sweep(Consts c, const R* __restrict__ Uin, const R* __restrict__ Pst,
                                                    R* __restrict__ Uout, Dyn* __restrict__ dyn, TvdArgs ta,
-                                                   TvdDiag<R> dg, Rem<R>* __restrict__ Cc) {
+                                                   TvdDiag<R> dg, const Rem<R>* Ci, Rem<R>* Co) {
   const Geom& g = c.g;
   if (dyn->err) return;
   if (ta.only_two_half && !dyn->two_half) return;   // second half pass not taken this step
@@ -1186,8 +1190,8 @@ __global__ void __launch_bounds__(128, TvdBlocks<R>::pencil) k_tvd_sweep(Consts 
         const int ci = DIR == 0 ? pos : aa, cj = DIR == 1 ? pos : (DIR == 0 ? aa : bb), ck = DIR == 2 ? pos : bb;
         const int sj = wrap_interior(cj, g.ny), sk = wrap_interior(ck, g.nz);
         const long long src = (long long)ci + (long long)g.sx * ((long long)sj + (long long)g.sy * sk);
-        cin = Cc + src;
-        if (sj == cj && sk == ck) cout = Cc + id;
+        cin = Ci + src;
+        if (sj == cj && sk == ck) cout = Co + id;
       }
       tvd_update<R, DIAG>(c, dtt, F0, Fm, q0, qm, c0, uc, u, &dg, id, qv0, qvm, cin, cout);
       if (!half_images) {
@@ -1220,7 +1224,7 @@ __device__ __forceinline__ R shfl(R v, int src) { return __shfl_sync(0xffffffffu
 template <class R, bool COMP = false>
 __global__ void __launch_bounds__(128, TvdBlocks<R>::lanes) k_tvd_sweep_xlanes(Consts c, const R* __restrict__ Uin, const R* __restrict__ Pst,
                                                           R* __restrict__ Uout, Dyn* __restrict__ dyn, int only_two_half,
-                                                          Rem<R>* __restrict__ Cc) {
+                                                          const Rem<R>* Ci, Rem<R>* Co) {
   const Geom& g = c.g;
   if (dyn->err) return;
   if (only_two_half && !dyn->two_half) return;
@@ -1282,8 +1286,8 @@ __global__ void __launch_bounds__(128, TvdBlocks<R>::lanes) k_tvd_sweep_xlanes(C
     Rem<R>* cout = nullptr;
     if (COMP) {  // FP32 compensated: the remainders of the interior cell this one is or images
       const int sj = wrap_interior((int)j, g.ny), sk = wrap_interior((int)k, g.nz);
-      cin = Cc + ((long long)g.sx * ((long long)sj + (long long)g.sy * sk) + pos);
-      if (sj == (int)j && sk == (int)k) cout = Cc + id;
+      cin = Ci + ((long long)g.sx * ((long long)sj + (long long)g.sy * sk) + pos);
+      if (sj == (int)j && sk == (int)k) cout = Co + id;
     }
     tvd_update<R>(c, dtt, F, Fm, qr, qm, c0, uc, u, nullptr, 0, (R)0, (R)0, cin, cout);
 #pragma unroll

@@ -49,7 +49,8 @@ struct Launch {
   // then ends the step
   // dg (per-routine TVDlimit on an output step): the diagnostics, through the
   // pencil kernel in every direction
-  // Cc (FP32 compensated fused steps, else null): the state's rounding remainders
+  // Cc (FP32 compensated fused steps, else null): the state's rounding remainders,
+  // two arrays of 8N: the current ones, and the x sweep's output
   static void tvd(const Consts& c, int dir, int mode, int only_two_half, const R* Uin, const R* Pst, R* Uout,
                   Dyn* dyn, cudaStream_t s, int td = 0, const TvdDiag<R>* dg = nullptr, Rem<R>* Cc = nullptr);
   // Clean_divB on U (phi, divb: N each); returns the number of launches
@@ -311,11 +312,15 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
   const int block = 128;
   const long long blocks = (total + block - 1) / block;
   if (dg) {
-    if (dir == 0) k_tvd_sweep<R, 0, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr);
-    else if (dir == 1) k_tvd_sweep<R, 1, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr);
-    else k_tvd_sweep<R, 2, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr);
+    if (dir == 0) k_tvd_sweep<R, 0, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
+    else if (dir == 1) k_tvd_sweep<R, 1, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
+    else k_tvd_sweep<R, 2, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
     return;
   }
+  // compensated: the remainders go to the second array in x, back in y, and stay in place in z
+  Rem<R>* const C2 = Cc ? Cc + 8 * g.N : nullptr;
+  const Rem<R>* const Ci = dir == 1 ? C2 : Cc;
+  Rem<R>* const Co = dir == 0 ? C2 : Cc;
   // contiguous x pencils: one cell per lane, 28 updates per warp, grid-stride
   // over a few waves of resident blocks
   const long long warps = (long long)g.sy * g.sz * ((g.nx + 27) / 28);
@@ -326,9 +331,9 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
       // at least one warp per segment (28 cells)
       const long long least = ((g.nx + 27) / 28 + 3) / 4;
       if (nb < least) nb = least;
-      if (dir == 0) (Cc ? k_tvd_xlanes_f32<true> : k_tvd_xlanes_f32<false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Cc);
-      else if (dir == 1) (Cc ? k_tvd_pencil_f32<1, true> : k_tvd_pencil_f32<1, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Cc);
-      else (Cc ? k_tvd_pencil_f32<2, true> : k_tvd_pencil_f32<2, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Cc);
+      if (dir == 0) (Cc ? k_tvd_xlanes_f32<true> : k_tvd_xlanes_f32<false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Ci, Co);
+      else if (dir == 1) (Cc ? k_tvd_pencil_f32<1, true> : k_tvd_pencil_f32<1, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Ci, Co);
+      else (Cc ? k_tvd_pencil_f32<2, true> : k_tvd_pencil_f32<2, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Ci, Co);
       return;
     }
   }
@@ -338,11 +343,11 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
     // every cell once (the lane kernel 32 for 28), is the faster one although its
     // loads are not coalesced (3.51 against 3.87 ms at 128 x 192 x 192)
     if constexpr (sizeof(R) == 8)
-      k_tvd_sweep<R, 0, false, false><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
+      k_tvd_sweep<R, 0, false, false><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Ci, Co);
     else
-      (Cc ? k_tvd_sweep_xlanes<R, true> : k_tvd_sweep_xlanes<R, false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Cc);
-  } else if (dir == 1) (Cc ? k_tvd_sweep<R, 1, false, true> : k_tvd_sweep<R, 1, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
-  else (Cc ? k_tvd_sweep<R, 2, false, true> : k_tvd_sweep<R, 2, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Cc);
+      (Cc ? k_tvd_sweep_xlanes<R, true> : k_tvd_sweep_xlanes<R, false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Ci, Co);
+  } else if (dir == 1) (Cc ? k_tvd_sweep<R, 1, false, true> : k_tvd_sweep<R, 1, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Ci, Co);
+  else (Cc ? k_tvd_sweep<R, 2, false, true> : k_tvd_sweep<R, 2, false, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, nod, Ci, Co);
 }
 
 template <class R>

@@ -323,7 +323,7 @@ template <int DIR, bool COMP>
 __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, const float* __restrict__ Uin,
                                                            const float* __restrict__ Pst, float* __restrict__ Uout,
                                                            Dyn* __restrict__ dyn, TvdArgs ta,
-                                                           Rem<float>* __restrict__ Cc) {
+                                                           const Rem<float>* Ci, Rem<float>* Co) {
   using namespace tvdf;
   if (dyn->err) return;
   if (ta.only_two_half && !dyn->two_half) return;  // second half pass not taken this step
@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
     Rem<float>* cout = nullptr;
     if (COMP) {  // the remainders of the interior cell this one is or images
       const int sj = wrap_interior(cj, g.ny), sk = wrap_interior(ck, g.nz);
-      cin = Cc + cidx32(g, aa, sj, sk);
-      if (sj == cj && sk == ck) cout = Cc + cidx32(g, aa, cj, ck);
+      cin = Ci + cidx32(g, aa, sj, sk);
+      if (sj == cj && sk == ck) cout = Co + cidx32(g, aa, cj, ck);
     }
     update(k, F, Fm, q, qm, a, uc, u, cin, cout, N);
     if (!half_images) store8(Uout, N, off, u);
@@ -412,7 +412,7 @@ template <bool COMP>
 __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, const float* __restrict__ Uin,
                                                            const float* __restrict__ Pst, float* __restrict__ Uout,
                                                            Dyn* __restrict__ dyn, int only_two_half,
-                                                           Rem<float>* __restrict__ Cc) {
+                                                           const Rem<float>* Ci, Rem<float>* Co) {
   using namespace tvdf;
   if (dyn->err) return;
   if (only_two_half && !dyn->two_half) return;
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, 
     if (COMP) {  // the remainders of the interior cell this one is or images
       const int kz = (int)(pen / (unsigned)g.sy), j = (int)pen - kz * g.sy;
       const int sj = wrap_interior(j, g.ny), sk = wrap_interior(kz, g.nz);
-      cin = Cc + cidx32(g, pos, sj, sk);
-      if (sj == j && sk == kz) cout = Cc + id;
+      cin = Ci + cidx32(g, pos, sj, sk);
+      if (sj == j && sk == kz) cout = Co + id;
     }
     float u[NV];
     update(k, F, Fm, q, qm, c0, uin, u, cin, cout, g.N);

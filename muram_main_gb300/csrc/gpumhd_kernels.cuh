@@ -772,10 +772,9 @@ __device__ __forceinline__ void tvd_cell(const Consts& c, const Raw9<R>& r, R hb
   cf = smax(cf, CME);
   cs2 *= cf * cf;
   t.cm = (R)0.0 + vv + d_sqrt(smax(cs2, lf * (cs2 + va2)));
-  if (mach) {
+  if (mach) {  // (not the field's diffusivity)
     t.he *= ((R)1.0 - CME);
     t.hv *= ((R)1.0 - CME);
-    t.hB *= ((R)1.0 - CME);
   }
   t.BC2 = (R)1.0 - lf;
   t.hd = (R)0;

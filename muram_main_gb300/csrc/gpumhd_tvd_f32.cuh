@@ -140,11 +140,10 @@ __device__ __forceinline__ void cell_of(const KC<float>& k, const Raw9<float>& r
   t.hv = fmaf(rf, p.v1, p.v0);
   t.hB = fmaf(rf, p.b1, p.b0);
   float CME = 0.0f;
-  if (k.CZ != 1.0f) {  // Mach-number damping above the photosphere
+  if (k.CZ != 1.0f) {  // Mach-number damping above the photosphere, not of the field's diffusivity
     CME = (1.0f - k.CZ) * ((float)(vabs >= k.CME_thresh * sqrt_(va2 + cs2)));
     t.he *= 1.0f - CME;
     t.hv *= 1.0f - CME;
-    t.hB *= 1.0f - CME;
   }
   cf = fmaxf(cf, CME);
   cs2 *= cf * cf;

@@ -16,8 +16,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 REF_BIN = os.path.join(HERE, "_ref", "muram_ref_harness")
 DROPIN_BIN = os.path.join(HERE, "_ref", "muram_gpu_dropin")
 # the reference sources: $MURAM_REF, else a checkout named "reference" beside
-# this repository
+# this repository; empty where there are none (a folder without src/ counts as none)
 REF_ROOT = os.environ.get("MURAM_REF") or os.path.normpath(os.path.join(HERE, "..", "..", "reference"))
+if not os.path.isdir(os.path.join(REF_ROOT, "src")):
+    REF_ROOT = ""
 
 
 def available():

@@ -12,6 +12,7 @@
 
 #include "../../include/gpumhd.h"
 #include "gpumhd_adjoint.cuh"
+#include "gpumhd_hostmem.cuh"
 #include "gpumhd_launch.cuh"
 
 using namespace gpumhd;
@@ -849,18 +850,44 @@ static long long host_nodes(const gpumhd_ctx* ctx) {
   return (long long)g.wx * g.sy * g.sz;
 }
 
+typedef CUresult (*PointerAttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+
+static PointerAttributeFn pointer_attribute_fn() {
+  static const PointerAttributeFn fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<PointerAttributeFn>(f);
+  }();
+  return fn;
+}
+
 // A kernel's address of pinned host memory [p, p + bytes), or null: pageable
-// memory, or a range that is not one pinned piece (those go through a staging
-// buffer).
-static void* pinned_on_device(const void* p, size_t bytes) {
-  cudaPointerAttributes a, b;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, (const char*)p + bytes - 1) != cudaSuccess) {
+// memory, a range that is not within one pinned piece, or (write) one the device
+// may only read (those go through a staging buffer).  The driver is asked for
+// the piece the first byte belongs to: two pieces registered apart keep their
+// distance on the device too, so their ends do not tell of a gap between them.
+static void* pinned_on_device(const void* p, size_t bytes, bool write) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
-      (char*)b.devicePointer != (char*)a.devicePointer + (bytes - 1))
+  const PointerAttributeFn get = pointer_attribute_fn();
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer || !get) return nullptr;
+  const CUdeviceptr d = (CUdeviceptr)a.devicePointer;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS || !hostmem::covers(start, size, d, bytes))
+    return nullptr;
+  unsigned access = CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+  if (write && get(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, d) == CUDA_SUCCESS &&
+      access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE)
     return nullptr;
   return a.devicePointer;
 }
@@ -875,7 +902,7 @@ static int upload_impl(gpumhd_ctx* ctx, int which, const H* host) {
   if (rc) return fail(ctx, rc, "upload: bad field %d", which);
   const long long N = host_nodes(ctx);
   const Geom& g = ctx->c.g;
-  const H* src = (const H*)pinned_on_device(host, sizeof(H) * nf * N);
+  const H* src = (const H*)pinned_on_device(host, sizeof(H) * nf * N, false);
   const bool direct = src != nullptr;
   if (!direct) {
     rc = ensure_staging(ctx);
@@ -1010,7 +1037,7 @@ static int download_impl(gpumhd_ctx* ctx, int which, H* host) {
   void* src = field_ptr(ctx, which, &nf, &rc);
   if (rc) return fail(ctx, rc, "download: bad field %d", which);
   const long long N = host_nodes(ctx);
-  H* dst = (H*)pinned_on_device(host, sizeof(H) * nf * N);
+  H* dst = (H*)pinned_on_device(host, sizeof(H) * nf * N, true);
   const bool direct = dst != nullptr;
   if (!direct) {
     rc = ensure_staging(ctx);

@@ -866,12 +866,15 @@ static PointerAttributeFn pointer_attribute_fn() {
   return fn;
 }
 
-// A kernel's address of pinned host memory [p, p + bytes), or null: pageable
-// memory, a range that is not within one pinned piece, or (write) one the device
-// may only read (those go through a staging buffer).  The driver is asked for
-// the piece the first byte belongs to: two pieces registered apart keep their
+// A kernel's address of `nodes` records of nf values of vsize bytes in pinned
+// host memory at p, or null: pageable memory, a range that is not within one
+// pinned piece, (write) one the device may only read, or records a kernel moves
+// slowly over the link (those go through a staging buffer).  The driver is asked
+// for the piece the first byte belongs to: two pieces registered apart keep their
 // distance on the device too, so their ends do not tell of a gap between them.
-static void* pinned_on_device(const void* p, size_t bytes, bool write) {
+static void* pinned_on_device(const void* p, int nf, int vsize, long long nodes, bool write) {
+  if (!hostmem::moves_directly(nf, vsize, (uint64_t)p, write)) return nullptr;
+  const size_t bytes = (size_t)vsize * nf * nodes;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
@@ -902,7 +905,7 @@ static int upload_impl(gpumhd_ctx* ctx, int which, const H* host) {
   if (rc) return fail(ctx, rc, "upload: bad field %d", which);
   const long long N = host_nodes(ctx);
   const Geom& g = ctx->c.g;
-  const H* src = (const H*)pinned_on_device(host, sizeof(H) * nf * N, false);
+  const H* src = (const H*)pinned_on_device(host, nf, sizeof(H), N, false);
   const bool direct = src != nullptr;
   if (!direct) {
     rc = ensure_staging(ctx);
@@ -1037,7 +1040,7 @@ static int download_impl(gpumhd_ctx* ctx, int which, H* host) {
   void* src = field_ptr(ctx, which, &nf, &rc);
   if (rc) return fail(ctx, rc, "download: bad field %d", which);
   const long long N = host_nodes(ctx);
-  H* dst = (H*)pinned_on_device(host, sizeof(H) * nf * N, true);
+  H* dst = (H*)pinned_on_device(host, nf, sizeof(H), N, true);
   const bool direct = dst != nullptr;
   if (!direct) {
     rc = ensure_staging(ctx);

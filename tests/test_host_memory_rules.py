@@ -10,6 +10,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = r"""
 #include "gpumhd_hostmem.cuh"
 extern "C" int covers(uint64_t s, uint64_t n, uint64_t p, uint64_t b) { return hostmem::covers(s, n, p, b); }
+extern "C" int moves_directly(int nf, int s, uint64_t a, int d) { return hostmem::moves_directly(nf, s, a, d != 0); }
 """
 
 
@@ -21,6 +22,7 @@ def rules(tmp_path_factory):
                     os.path.join(ROOT, "muram_main_gb300", "csrc"), str(d / "r.cpp"), "-o", str(d / "r.so")], check=True)
     lib = C.CDLL(str(d / "r.so"))
     lib.covers.argtypes = [C.c_uint64] * 4
+    lib.moves_directly.argtypes = [C.c_int, C.c_int, C.c_uint64, C.c_int]
     return lib
 
 
@@ -44,3 +46,15 @@ def test_two_pieces_with_a_gap(rules):
 
 def test_nothing_is_covered_by_an_unknown_piece(rules):
     assert not rules.covers(0, 0, 0x7f0000000000, 8)
+
+
+@pytest.mark.parametrize("size", [4, 8])
+@pytest.mark.parametrize("download", [0, 1])
+def test_records_move_directly_only_in_whole_pieces(rules, size, download):
+    """Unaligned records go through the staging buffer, but for float uploads."""
+    at = 0x7f0000000000
+    assert all(rules.moves_directly(8, size, at + 16 * k, download) for k in range(4))
+    assert all(rules.moves_directly(8, size, at + k, download) == (size == 4 and not download)
+               for k in (4, 8, 12, 20, 24))
+    assert all(rules.moves_directly(1, size, at + k, download) for k in (0, 4, 8, 16))
+    assert not rules.moves_directly(3, size, at, download)

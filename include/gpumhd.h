@@ -270,9 +270,11 @@ int gpumhd_tile_from(gpumhd_ctx* ctx, gpumhd_ctx* src);
 
 /* ---- launch shapes (no counterpart in the reference: GPU tiling only) ----
  * stage_zchunk: z planes per stage-kernel block (0: chosen from the GPU's
- * occupancy); tvd_chunk: cells per thread of the y / z TVD sweeps (0: up to 32,
- * fewer on boxes that do not fill the GPU).
- * Results do not depend on them. */
+ * occupancy); tvd_chunk: the most cells per thread of the y / z TVD sweeps (0:
+ * 32): a box that steps alone and does not fill the GPU takes fewer, in an
+ * ensemble, whose other boxes fill it, a chunk other than 0 is taken as it is.
+ * What gpumhd_get_tuning returns, set here on another context, gives it the same
+ * shapes.  Results do not depend on them. */
 int gpumhd_set_tuning(gpumhd_ctx* ctx, int stage_zchunk, int tvd_chunk);
 /* Test hook of the TMA stage kernel's bounded waits (no counterpart in the
  * reference; for testing the error path only).  wait_cycles limits each wait

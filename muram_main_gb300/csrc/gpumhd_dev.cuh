@@ -394,7 +394,7 @@ struct C2POut {
 
 // Full ConsToPrim arithmetic for one cell given primitives (src/cons_to_prim.C:148-243).
 __device__ inline C2POut c2p_eos_full(const Consts& c, double d, double ei, double dn) {
-  const double eps = ei * dn + c.eps_off;
+  const double eps = mad(ei, dn, c.eps_off);
   const double lgr = d_log(d);
   const double ep = d_log(eps);
   const double lr = lgr;
@@ -419,9 +419,9 @@ __device__ inline C2POut c2p_eos_full(const Consts& c, double d, double ei, doub
     if (t == 2) { out[t] = 0.0; continue; }
     const float* T = c.tab[t];
     double s = c0 * i64f::from_float(T[a11]);
-    s += c1 * i64f::from_float(T[a10]);
-    s += c2 * i64f::from_float(T[a01]);
-    s += c3 * i64f::from_float(T[a00]);
+    s = mad(c1, i64f::from_float(T[a10]), s);
+    s = mad(c2, i64f::from_float(T[a01]), s);
+    s = mad(c3, i64f::from_float(T[a00]), s);
     out[t] = d_exp(s);
   }
   double pr = out[0], tm = out[1], nl = out[3];

@@ -426,9 +426,10 @@ __device__ __forceinline__ R boris_lf(const R* cen, R inv_va2max) {
 
 // Sources and semi-relativistic (Boris) correction added to the residual Racc
 // of a cell with primitives cen (src/Add_Sources_Integrate_SR.C:331-392):
-// gravity along x, the radiative term (zero here), then the correction.
+// gravity along x, the radiative term (zero here), then the correction, whose
+// energy b3_out receives.
 template <class R>
-__device__ __forceinline__ void stage_sources(R* Racc, const R* cen, R gx, R inv_va2max, R invRdt) {
+__device__ __forceinline__ void stage_sources(R* Racc, const R* cen, R gx, R inv_va2max, R invRdt, R* b3_out = nullptr) {
   const R rh = cen[P_D], vx = cen[P_V1], vy = cen[P_V2], vz = cen[P_V3];
   const R bx = cen[P_B1], by = cen[P_B2], bz = cen[P_B3];
   // the radiative term is zero times dn / max(dn, 0), dn the radiative limit
@@ -456,6 +457,7 @@ __device__ __forceinline__ void stage_sources(R* Racc, const R* cen, R gx, R inv
   Racc[2] += b1;
   Racc[3] += b2;
   Racc[4] += b3;
+  if (b3_out) *b3_out = b3;
 }
 
 // Shared memory of one stage block: the x fluxes of (TX+4) x TY cells, the y
@@ -1487,13 +1489,14 @@ __global__ void __launch_bounds__(256) k_diag_residual(Consts c, const R* __rest
       const R Bd1 = cen[P_B1 + D1];
       const R Bd2 = cen[P_B1 + Dirs<D1>::d2], Bd3 = cen[P_B1 + Dirs<D1>::d3];
       R cbb[3];
-      cbb[D1] = -Bd2 * dB2 - Bd3 * dB3;
+      cbb[D1] = nmad(Bd3, dB3, -Bd2 * dB2);
       cbb[Dirs<D1>::d2] = Bd1 * dB2;
       cbb[Dirs<D1>::d3] = Bd1 * dB3;
-      const R lrt0 = lf * Dq[7] + ((R)1.0 - lf) * cbb[0];
-      const R lrt1 = lf * Dq[8] + ((R)1.0 - lf) * cbb[1];
-      const R lrt2 = lf * Dq[9] + ((R)1.0 - lf) * cbb[2];
-      t3 += cen[P_V1] * lrt0 + cen[P_V2] * lrt1 + cen[P_V3] * lrt2;
+      const R lc = (R)1.0 - lf;
+      const R lrt0 = mad(lf, Dq[7], lc * cbb[0]);
+      const R lrt1 = mad(lf, Dq[8], lc * cbb[1]);
+      const R lrt2 = mad(lf, Dq[9], lc * cbb[2]);
+      t3 += dot3(cen[P_V1], lrt0, cen[P_V2], lrt1, cen[P_V3], lrt2);
     };
     direction(std::integral_constant<int, 0>());
     direction(std::integral_constant<int, 1>());
@@ -1582,35 +1585,22 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_source_integrate(Consts
     R r[NV], u[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) { r[v] = Res[(unsigned)v * N + id]; u[v] = U[(unsigned)v * N + id]; }
-    R dn = invRdt * u[4];
-    R efaci = d_div(dn, d_fmax(dn, (R)0.0));
-    dn = kc<R>(c).gx * u[0] - (R)0.0;
-    R edmp = dn * u[1];
-    r[1] += dn;
-    r[4] += edmp + (R)0.0 * efaci;
-    const R rh = u[0], rd = r[0], vx = u[1], vy = u[2], vz = u[3], bx = u[5], by = u[6], bz = u[7];
-    R fx = r[1], fy = r[2], fz = r[3];
-    const R bb = bx * bx + by * by + bz * bz;
-    const R va2 = d_div(bb, rh);
-    const R x2 = va2 * inv_va2max, x4 = x2 * x2;
-    const R bf = d_div(x4, (R)1 + x2 + x4);
-    fx -= vx * rd;
-    fy -= vy * rd;
-    fz -= vz * rd;
-    const R q = d_div(fx * bx + fy * by + fz * bz, d_fmax(tiny100<R>(), bb));
-    const R b0 = -bf * (fx - q * bx), b1 = -bf * (fy - q * by), b2 = -bf * (fz - q * bz);
-    const R b3 = b0 * vx + b1 * vy + b2 * vz;
-    r[1] += b0; r[2] += b1; r[3] += b2; r[4] += b3;
-    R un[NV];
+    // the fused stage's sources and update, so that both round alike
+    R cen[NPRIM];  // its first eight are a primitive state's fields, the only ones read here
 #pragma unroll
-    for (int v = 0; v < NV; v++) un[v] = U0[(unsigned)v * N + id] + wdt * r[v];
+    for (int v = 0; v < NV; v++) cen[v] = u[v];
+    R b3, un[NV];
+    stage_sources<R>(r, cen, kc<R>(c).gx, inv_va2max, invRdt, &b3);
+#pragma unroll
+    for (int v = 0; v < NV; v++) un[v] = mad(wdt, r[v], U0[(unsigned)v * N + id]);
     // Res is zero for the next MHD_Residual: the host marks it so and the
     // next residual writes it without reading it (no pass stores the zeros)
     const R ee = un[4];
     tcheck_cell<R>(c, vmax, emax, un[0], un[1], un[2], un[3], un[4]);
     if (diag) {
-      diag[3 * N + id] = efaci;
-      diag[4 * N + id] = edmp;
+      const R dn = invRdt * u[4];
+      diag[3 * N + id] = (dn > (R)0 && dn < (R)INFINITY) ? (R)1.0 : d_div(dn, d_fmax(dn, (R)0.0));
+      diag[4 * N + id] = kc<R>(c).gx * u[0] * u[1];
       diag[5 * N + id] = b3;
       diag[6 * N + id] += (un[4] - ee) * invdt;
     }

@@ -15,7 +15,9 @@
 // Adjoint fields live on the interior only (nx*ny*nz per variable, x fastest)
 // with periodic neighbours; forward fields are the ghost-filled arrays the
 // forward kernels wrote.  Compiled without FMA contraction like the FP64
-// forward kernels, so the recomputed forward values equal the forward run's.
+// forward kernels, and recomputing with their formulas, fused where those are
+// (mad, nmad, dot3), so the recomputed forward values equal the forward run's to
+// the bit and a clamp at a tie takes the branch the forward took.
 #include "gpumhd_adjoint.cuh"
 #include "gpumhd_dual.cuh"
 
@@ -59,12 +61,12 @@ __device__ __forceinline__ void apply_direction_rev(const double* Dq, const doub
   const double dB2 = Dq[10], dB3 = Dq[11];
   const double Bd1 = cen[P_B1 + D1], Bd2 = cen[P_B1 + d2], Bd3 = cen[P_B1 + d3];
   double cbb[3];
-  cbb[D1] = -Bd2 * dB2 - Bd3 * dB3;
+  cbb[D1] = nmad(Bd3, dB3, -Bd2 * dB2);
   cbb[d2] = Bd1 * dB2;
   cbb[d3] = Bd1 * dB3;
   double l_cbb[3];
   for (int i = 0; i < 3; i++) {  // lrt_i = lf*Dq[7+i] + (1-lf)*cbb_i; res[1+i] += lrt_i; res[4] += v_i*lrt_i
-    const double lrt = lf * Dq[7 + i] + (1.0 - lf) * cbb[i];
+    const double lrt = mad(lf, Dq[7 + i], (1.0 - lf) * cbb[i]);
     const double l_lrt = lR[1 + i] + lR[4] * cen[P_V1 + i];
     l_cen[P_V1 + i] += lR[4] * lrt;
     l_dq[7 + i] = l_lrt * lf;
@@ -92,19 +94,19 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
   const double rh = cen[P_D];
   const double v[3] = {cen[P_V1], cen[P_V2], cen[P_V3]}, B[3] = {cen[P_B1], cen[P_B2], cen[P_B3]};
   // ---- forward
-  const double dn2 = gx * rh - 0.0;
+  const double dn2 = gx * rh;
   const double F[3] = {R[1] + dn2, R[2], R[3]};
   const double rd = R[0];
-  const double bb = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
+  const double bb = dot3(B[0], B[0], B[1], B[1], B[2], B[2]);
   const double va2 = d_div(bb, rh);
   const double x2 = va2 * inv_va2max, x4 = x2 * x2;
   const double D = 1.0 + x2 + x4;
   const double bf = d_div(x4, D);
   double f[3], bo[3];
-  for (int i = 0; i < 3; i++) f[i] = F[i] - v[i] * rd;
+  for (int i = 0; i < 3; i++) f[i] = nmad(v[i], rd, F[i]);
   const double bq = d_fmax(tiny, bb);
-  const double q = d_div(f[0] * B[0] + f[1] * B[1] + f[2] * B[2], bq);
-  for (int i = 0; i < 3; i++) bo[i] = -bf * (f[i] - q * B[i]);
+  const double q = d_div(dot3(f[0], B[0], f[1], B[1], f[2], B[2]), bq);
+  for (int i = 0; i < 3; i++) bo[i] = -bf * nmad(q, B[i], f[i]);
   // ---- reverse
   double l_v[3] = {0.0, 0.0, 0.0}, l_B[3] = {0.0, 0.0, 0.0}, l_f[3];
   double l_bf = 0.0, l_q = 0.0;
@@ -156,10 +158,10 @@ __device__ __forceinline__ void stage_sources_rev(const double* R, const double*
 __device__ __forceinline__ void boris_lf_rev(const double* cen, double inv_va2max, double l_lf, double* l_cen) {
   const double dn = d_div(1.0, cen[P_D]);
   const double B[3] = {cen[P_B1], cen[P_B2], cen[P_B3]};
-  const double bb = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
+  const double bb = dot3(B[0], B[0], B[1], B[1], B[2], B[2]);
   const double va2 = bb * dn;
-  const double x2 = va2 * inv_va2max, x4 = x2 * x2, s = 1.0 + x2;
-  const double E = s + x4, lf = d_div(s, E);
+  const double x2 = va2 * inv_va2max, s = 1.0 + x2;
+  const double E = mad(x2, x2, s), lf = d_div(s, E);
   const double l_s = d_div(l_lf * (1.0 - lf), E);  // lf = s / (s + x4)
   const double l_x4 = d_div(-l_lf * lf, E);
   const double l_x2 = l_s + l_x4 * 2.0 * x2;
@@ -220,7 +222,7 @@ __device__ __forceinline__ void prim_of_raw_rev(const Raw9<double>& r, const dou
   const double m[3] = {r.v[1], r.v[2], r.v[3]};
   double v[3];
   for (int t = 0; t < 3; t++) v[t] = m[t] * dn;
-  const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+  const double vv = dot3(v[0], v[0], v[1], v[1], v[2], v[2]);
   double l_d = lw[P_D] + lw[P_EK] * 0.5 * vv;  // ekin = 0.5 * d * vv
   double l_vv = lw[P_EK] * 0.5 * d;
   const double l_e = lw[P_EI];  // ei = e - 0.5 * vv * d
@@ -296,7 +298,7 @@ __global__ void k_stage_a(Consts c, const Dyn* dyn, Box b, const double* __restr
     double pre[NV], lo[NV];
 #pragma unroll
     for (int q = 0; q < NV; q++) {
-      pre[q] = U0[(long long)q * g.N + id] + wdt * G[q];
+      pre[q] = mad(wdt, G[q], U0[(long long)q * g.N + id]);
       lo[q] = lam_out[(long long)q * b.n + li];
     }
     // Tcheck (density, momentum, energy) transposed; the field passes through
@@ -497,7 +499,7 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
     den[v] = smax(tiny, fabs(sl[v]));
     rf[v] = d_div(fabs(sll[v]), den[v]);
     cfv[v] = smax(0.0, smin(sll[v], sl[v])) + smin(0.0, smax(sll[v], sl[v]));
-    G[v] = smax(0.0, 1.0 + dnv * (rf[v] - 1.0));
+    G[v] = smax(0.0, mad(dnv, rf[v] - 1.0, 1.0));
     F0[v] = G[v] * cfv[v];
   }
   const double M = smax(a.cm, b.cm);
@@ -543,8 +545,8 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
   const double CZ = smin(k.CZ, k.CZ);
   const double mcz = f0 * CZ;
   double fn[4];
-  for (int t = 1; t <= 3; t++) fn[t] = F[t] * U0 + u[t] * mcz;
-  const double S = u[1] * fn[1] + u[2] * fn[2] + u[3] * fn[3];
+  for (int t = 1; t <= 3; t++) fn[t] = mad(u[t], mcz, F[t] * U0);
+  const double S = dot3(u[1], fn[1], u[2], fn[2], u[3], fn[3]);
   const bool zero5 = DIR == 0 && !c.g.periodic_x && (ia == sz - GH - 1 || ia == GH - 1);
   const double Fq[3] = {zero5 ? 0.0 : F[5], F[6], F[7]};
   // ---- reverse
@@ -640,7 +642,7 @@ __device__ void tvd_flux_rev(const Consts& c, const TCell<double>& am, const TCe
     const int df = dn_field(v);
     const double dnv = tf(a)[df];
     double l_rf = 0.0;
-    if (0.0 < 1.0 + dnv * (rf[v] - 1.0)) {  // G = max(0, 1 + dn*(rf - 1))
+    if (0.0 < mad(dnv, rf[v] - 1.0, 1.0)) {  // G = max(0, 1 + dn*(rf - 1))
       l_a[df] += l_G * (rf[v] - 1.0);
       l_rf = l_G * dnv;
     }
@@ -679,23 +681,23 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
   const double W = res[1] * c0.q[1] + res[2] * c0.q[2] + res[3] * c0.q[3];
   const double r4a = res[4] + (1.0 - c0.qt) * W;
   const double bs = smax(tiny, c0.bsqr);
-  const double num = res[1] * c0.q[5] + res[2] * c0.q[6] + res[3] * c0.q[7];
+  const double num = dot3(res[1], c0.q[5], res[2], c0.q[6], res[3], c0.q[7]);
   const double dn = d_div(num, bs);
   double bb[3];
-  for (int t = 0; t < 3; t++) bb[t] = -c0.BC2 * (res[1 + t] - dn * c0.q[5 + t]);
-  const double b3 = bb[0] * c0.q[1] + bb[1] * c0.q[2] + bb[2] * c0.q[3];
+  for (int t = 0; t < 3; t++) bb[t] = -c0.BC2 * nmad(dn, c0.q[5 + t], res[1 + t]);
+  const double b3 = dot3(bb[0], c0.q[1], bb[1], c0.q[2], bb[2], c0.q[3]);
   double r[NV];
 #pragma unroll
   for (int v = 0; v < NV; v++) r[v] = res[v];
   for (int t = 0; t < 3; t++) r[1 + t] += bb[t];
   const double qres = 0.5 * (qp + qm) * c0.qt;
-  r[4] = (r4a + b3) + dtt * qres;
+  r[4] = mad(dtt, qres, r4a + b3);
   double u[NV];
 #pragma unroll
   for (int v = 0; v < NV; v++) u[v] = u_in[v] + r[v];
   const double u0f = smax(k.rho_min, u[0]);
-  const double K = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
-  const double ef = k.eps_min * u0f + d_div(0.5 * K, u0f);
+  const double K = dot3(u[1], u[1], u[2], u[2], u[3], u[3]);
+  const double ef = mad(k.eps_min, u0f, d_div(0.5 * K, u0f));
   // ---- reverse
   double l_u[NV];
 #pragma unroll
@@ -726,7 +728,7 @@ __device__ void tvd_update_rev(const Consts& c, double dtt, const double* Fp, co
   }
   double l_dn = 0.0;
   for (int t = 0; t < 3; t++) {  // bb = -BC2 * (res - dn * qB)
-    const double in = res[1 + t] - dn * c0.q[5 + t];
+    const double in = nmad(dn, c0.q[5 + t], res[1 + t]);
     l_c0[T_BC2] -= l_bb[t] * in;
     const double l_inn = -c0.BC2 * l_bb[t];
     l_res[1 + t] += l_inn;
@@ -832,12 +834,12 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
   const double dn = d_div(1.0, d);
   double v[3], Bc[3];
   for (int t = 0; t < 3; t++) { v[t] = r.v[1 + t] * dn; Bc[t] = r.v[5 + t]; }
-  const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-  const double bb = Bc[0] * Bc[0] + Bc[1] * Bc[1] + Bc[2] * Bc[2];
-  const double e = r.v[4] * dn - 0.5 * vv;
+  const double vv = dot3(v[0], v[0], v[1], v[1], v[2], v[2]);
+  const double bb = dot3(Bc[0], Bc[0], Bc[1], Bc[1], Bc[2], Bc[2]);
+  const double e = mad(r.v[4], dn, -0.5 * vv);
   const double vs = d_sqrt(vv);
   const double va2 = bb * dn;
-  const double x2 = va2 * inv_va2max, x4 = x2 * x2, s = 1.0 + x2, E = s + x4;
+  const double x2 = va2 * inv_va2max, s = 1.0 + x2, E = mad(x2, x2, s);
   const double lf = d_div(s, E);
   const double cs2 = (5.0 / 3.0) * r.v[8] * dn;
   const double cfast = d_sqrt(va2 + cs2);
@@ -846,7 +848,9 @@ __device__ void tvd_cell_rev(const Consts& c, const Raw9<double>& r, double hb, 
   const double rl = d_div(d2, d2 + k.rho_lev);
   const double rf = smin(lf, rl);
   const double hh = 1.0 - hb - ht;
-  const double cfa = hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + (1.0 - rf) * k.tvd_cs[2]) * hh + ht * k.tvd_cs[3];
+  const double cfa = hb == 0.0 && ht == 0.0
+                         ? mad(rf, k.tvd_cs[1], (1.0 - rf) * k.tvd_cs[2])
+                         : hb * k.tvd_cs[0] + (rf * k.tvd_cs[1] + (1.0 - rf) * k.tvd_cs[2]) * hh + ht * k.tvd_cs[3];
   const double cf = smax(cfa, CME);
   const double cs2b = cs2 * (cf * cf);
   const double A = lf * (cs2b + va2);

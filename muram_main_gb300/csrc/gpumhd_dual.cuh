@@ -82,6 +82,18 @@ GPUMHD_DUAL_CMP(==)
 GPUMHD_DUAL_CMP(!=)
 #undef GPUMHD_DUAL_CMP
 
+// a * b + c and c - a * b, the values rounded once as the forward's
+template <int K> __device__ __forceinline__ Dual<K> mad(const Dual<K>& a, const Dual<K>& b, const Dual<K>& c) {
+  Dual<K> r;
+  r.v = mad(a.v, b.v, c.v);
+#pragma unroll
+  for (int k = 0; k < K; k++) r.d[k] = a.d[k] * b.v + a.v * b.d[k] + c.d[k];
+  return r;
+}
+template <int K> __device__ __forceinline__ Dual<K> nmad(const Dual<K>& a, const Dual<K>& b, const Dual<K>& c) {
+  return mad(-a, b, c);
+}
+
 template <int K> __device__ __forceinline__ Dual<K> dual_chain(const Dual<K>& a, double fv, double dfdx) {
   Dual<K> r;
   r.v = fv;
@@ -118,7 +130,7 @@ template <int K> __device__ __forceinline__ Dual<K> d_fmax(const Dual<K>& a, dou
 // c2p_eos_full's pressure.
 template <class R>
 __device__ __forceinline__ R eos_pres_t(const Consts& c, R d, R ei, R dn) {
-  const R eps = ei * dn + c.eps_off;
+  const R eps = mad(ei, dn, R(c.eps_off));
   const R lgr = d_log(d);
   const R ep = d_log(eps);
   int i_d = cvt_x86((val(lgr) - c.xlr0) * c.inv_del_lr);
@@ -135,9 +147,9 @@ __device__ __forceinline__ R eos_pres_t(const Consts& c, R d, R ei, R dn) {
   const long long r1 = (long long)(i_e + 1) * c.N_lr + i_d;
   const long long r0 = (long long)i_e * c.N_lr + i_d;
   R s = c0 * (double)T[r1 + 1];
-  s += c1 * (double)T[r1];
-  s += c2 * (double)T[r0 + 1];
-  s += c3 * (double)T[r0];
+  s = mad(c1, R((double)T[r1]), s);
+  s = mad(c2, R((double)T[r0 + 1]), s);
+  s = mad(c3, R((double)T[r0]), s);
   R pr = d_exp(s);
   if (val(lgr) < c.xlr0) pr = c.c_pres * ei;
   if (val(eps) > 0.8 * c.eps_max) {

@@ -1006,6 +1006,47 @@ __global__ void k_tvd_t1(Consts c, const Dyn* dyn, Box b, const double* __restri
   }
 }
 
+// The boundary profiles are functions of x that are not periodic: the x ghosts of
+// a periodic box carry the boundary's values (hb or ht = 1), so the interface at
+// -1/2 is not the image of the one at nx-1/2, nor a ghost's slope and cell
+// quantities those of the cell it images.  In the x sweep each is transposed for
+// itself: interface -1/2 (k_tvd_x2), the slopes of cells -1 and nx (k_tvd_x3) and
+// the cell quantities of the four ghosts (k_tvd_x4), one thread per pencil; y and
+// z sweeps wrap.
+
+// The flux of the interface between T[1] and T[2] (memory index p of T[1])
+// transposed in one reverse pass onto its four cells' TCells (am, a, b, bp: 19
+// each) and its two slopes (8 each): 92 values, out[f * stride].
+template <int DIR>
+__device__ __forceinline__ void interface_rev(const Consts& c, const Sweep& s, const TCell<double>* T, int p,
+                                              const double* lF, double* out, long long stride) {
+  double sa[NV], sb[NV];
+  tvd_slope<double>(c, T[0], T[1], T[2], s.vsqr_diff, sa);
+  tvd_slope<double>(c, T[1], T[2], T[3], s.vsqr_diff, sb);
+  double l_t[4][NT], l_s[2][NV];
+  for (int r = 0; r < 4; r++)
+    for (int f = 0; f < NT; f++) l_t[r][f] = 0.0;
+  for (int q = 0; q < NV; q++) l_s[0][q] = l_s[1][q] = 0.0;
+  tvd_flux_rev<DIR>(c, T[0], T[1], T[2], T[3], sa, sb, p, s.sz, s.fac0, s.cmax_t, s.hyper, s.istart, lF, lF[NV],
+                    l_t[0], l_t[1], l_t[2], l_t[3], l_s[0], l_s[1]);
+  for (int r = 0; r < 4; r++)
+    for (int f = 0; f < NT; f++) out[(r * NT + f) * stride] = l_t[r][f];
+  for (int r = 0; r < 2; r++)
+    for (int q = 0; q < NV; q++) out[(4 * NT + r * NV + q) * stride] = l_s[r][q];
+}
+
+// The slope of the middle cell transposed in one reverse pass onto its three
+// cells: 3 x 19 values, out[f * stride].
+__device__ __forceinline__ void slope_rev(const Consts& c, const Sweep& s, const TCell<double>* T, const double* ls,
+                                          double* out, long long stride) {
+  double l_t[3][NT];
+  for (int r = 0; r < 3; r++)
+    for (int f = 0; f < NT; f++) l_t[r][f] = 0.0;
+  tvd_slope_rev(c, T[0], T[1], T[2], s.vsqr_diff, ls, l_t[0], l_t[1], l_t[2]);
+  for (int r = 0; r < 3; r++)
+    for (int f = 0; f < NT; f++) out[(r * NT + f) * stride] = l_t[r][f];
+}
+
 // T2: per interface i+1/2 (stored at its left cell i), the interface flux
 // transposed onto its four cells' TCells (am, a, b, bp: 19 each) and its two
 // slopes (8 each): 92 values per interface.
@@ -1018,26 +1059,28 @@ __global__ void k_tvd_t2(Consts c, const Dyn* dyn, Box b, const double* __restri
     int i, j, k;
     ijk(b, li, i, j, k);
     const long long lr = nbr<DIR>(b, i, j, k, 1);
+    const bool last_x = DIR == 0 && i == b.nx - 1;  // cell 0's left flux is interface -1/2's
     double lF[NV + 1];
-    for (int q = 0; q <= NV; q++) lF[q] = i_fp[(long long)q * b.n + li] + i_fm[(long long)q * b.n + lr];
+    for (int q = 0; q <= NV; q++)
+      lF[q] = i_fp[(long long)q * b.n + li] + (last_x ? 0.0 : i_fm[(long long)q * b.n + lr]);
     TCell<double> T[4];
     for (int o = -1; o <= 2; o++) cell_load<DIR>(c.g, tc, i, j, k, o, T[o + 1]);
-    double sa[NV], sb[NV];
-    tvd_slope<double>(c, T[0], T[1], T[2], s.vsqr_diff, sa);
-    tvd_slope<double>(c, T[1], T[2], T[3], s.vsqr_diff, sb);
-    const int p = pos_of<DIR>(i, j, k);
-    // the interface flux transposed in one reverse pass onto its four cells'
-    // TCells (am, a, b, bp) and its two slopes
-    double l_t[4][NT], l_s[2][NV];
-    for (int r = 0; r < 4; r++)
-      for (int f = 0; f < NT; f++) l_t[r][f] = 0.0;
-    for (int q = 0; q < NV; q++) l_s[0][q] = l_s[1][q] = 0.0;
-    tvd_flux_rev<DIR>(c, T[0], T[1], T[2], T[3], sa, sb, p, s.sz, s.fac0, s.cmax_t, s.hyper, s.istart, lF, lF[NV],
-                      l_t[0], l_t[1], l_t[2], l_t[3], l_s[0], l_s[1]);
-    for (int r = 0; r < 4; r++)
-      for (int f = 0; f < NT; f++) o_if[(long long)(r * NT + f) * b.n + li] = l_t[r][f];
-    for (int r = 0; r < 2; r++)
-      for (int q = 0; q < NV; q++) o_if[(long long)(4 * NT + r * NV + q) * b.n + li] = l_s[r][q];
+    interface_rev<DIR>(c, s, T, pos_of<DIR>(i, j, k), lF, o_if + li, b.n);
+  }
+}
+// Interface -1/2 of the x sweep: 92 values per pencil.
+__global__ void k_tvd_x2(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
+                         const double* __restrict__ i_fm, double* __restrict__ o_xif) {
+  const Sweep s = sweep_of<0>(c, dyn);
+  const int np = b.ny * b.nz;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np; t += gridDim.x * blockDim.x) {
+    const int j = t % b.ny, k = t / b.ny;
+    const long long li = lin(b, 0, j, k);
+    double lF[NV + 1];
+    for (int q = 0; q <= NV; q++) lF[q] = i_fm[(long long)q * b.n + li];
+    TCell<double> T[4];
+    for (int o = -1; o <= 2; o++) cell_load<0>(c.g, tc, -1, j, k, o, T[o + 1]);
+    interface_rev<0>(c, s, T, pos_of<0>(-1, j, k), lF, o_xif + t, np);
   }
 }
 
@@ -1045,25 +1088,39 @@ __global__ void k_tvd_t2(Consts c, const Dyn* dyn, Box b, const double* __restri
 // (i-1: q; i: q, hb, ht, vsqr; i+1: q): 3 x 19 values.
 template <int DIR>
 __global__ void k_tvd_t3(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
-                         const double* __restrict__ i_if, double* __restrict__ o_sl) {
+                         const double* __restrict__ i_if, const double* __restrict__ i_xif, double* __restrict__ o_sl) {
   const Sweep s = sweep_of<DIR>(c, dyn);
+  const long long np = (long long)b.ny * b.nz;
   for (long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x; li < b.n;
        li += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     ijk(b, li, i, j, k);
     const long long ll = nbr<DIR>(b, i, j, k, -1);
+    const bool first_x = DIR == 0 && i == 0;
+    const double* const lb = first_x ? i_xif + (j + (long long)b.ny * k) : i_if + ll;  // the interface left of i
+    const long long sb = first_x ? np : b.n;
     double ls[NV];
-    for (int q = 0; q < NV; q++)
-      ls[q] = i_if[(long long)(4 * NT + q) * b.n + li] + i_if[(long long)(4 * NT + NV + q) * b.n + ll];
+    for (int q = 0; q < NV; q++) ls[q] = i_if[(long long)(4 * NT + q) * b.n + li] + lb[(4 * NT + NV + q) * sb];
     TCell<double> T[3];
     for (int o = -1; o <= 1; o++) cell_load<DIR>(c.g, tc, i, j, k, o, T[o + 1]);
-    // the slope transposed in one reverse pass onto its three cells
-    double l_t[3][NT];
-    for (int r = 0; r < 3; r++)
-      for (int f = 0; f < NT; f++) l_t[r][f] = 0.0;
-    tvd_slope_rev(c, T[0], T[1], T[2], s.vsqr_diff, ls, l_t[0], l_t[1], l_t[2]);
-    for (int r = 0; r < 3; r++)
-      for (int f = 0; f < NT; f++) o_sl[(long long)(r * NT + f) * b.n + li] = l_t[r][f];
+    slope_rev(c, s, T, ls, o_sl + li, b.n);
+  }
+}
+// The slopes of cells -1 and nx of the x sweep: 2 x 57 values per pencil.
+__global__ void k_tvd_x3(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
+                         const double* __restrict__ i_if, const double* __restrict__ i_xif,
+                         double* __restrict__ o_xsl) {
+  const Sweep s = sweep_of<0>(c, dyn);
+  const int np = b.ny * b.nz;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * np; t += gridDim.x * blockDim.x) {
+    const int end = t / np, pen = t - end * np, j = pen % b.ny, k = pen / b.ny;
+    const long long last = lin(b, b.nx - 1, j, k);
+    double ls[NV];
+    for (int q = 0; q < NV; q++)
+      ls[q] = end == 0 ? i_xif[(long long)(4 * NT + q) * np + pen] : i_if[(long long)(4 * NT + NV + q) * b.n + last];
+    TCell<double> T[3];
+    for (int o = -1; o <= 1; o++) cell_load<0>(c.g, tc, end == 0 ? -1 : b.nx, j, k, o, T[o + 1]);
+    slope_rev(c, s, T, ls, o_xsl + (long long)end * 3 * NT * np + pen, np);
   }
 }
 
@@ -1074,6 +1131,7 @@ template <int DIR>
 __global__ void k_tvd_t4(Consts c, const Dyn* dyn, Box b, const double* __restrict__ V, const double* __restrict__ P,
                          const double* __restrict__ i_in, const double* __restrict__ i_cell,
                          const double* __restrict__ i_if, const double* __restrict__ i_sl,
+                         const double* __restrict__ i_xif, const double* __restrict__ i_xsl,
                          double* __restrict__ lam_in, double* __restrict__ lam_p) {
   const Sweep s = sweep_of<DIR>(c, dyn);
   for (long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x; li < b.n;
@@ -1081,16 +1139,27 @@ __global__ void k_tvd_t4(Consts c, const Dyn* dyn, Box b, const double* __restri
     int i, j, k;
     ijk(b, li, i, j, k);
     const long long m1 = nbr<DIR>(b, i, j, k, -1), m2 = nbr<DIR>(b, i, j, k, -2), p1 = nbr<DIR>(b, i, j, k, 1);
+    const long long np = (long long)b.ny * b.nz, pen = j + (long long)b.ny * k;
     double lt[NT];
     for (int f = 0; f < NT; f++) {
       double a = i_cell[(long long)f * b.n + li];
-      a += i_if[(long long)(1 * NT + f) * b.n + li];   // as a of interface j+1/2
-      a += i_if[(long long)(2 * NT + f) * b.n + m1];   // as b of interface j-1/2
-      a += i_if[(long long)(0 * NT + f) * b.n + p1];   // as am of interface j+3/2
-      a += i_if[(long long)(3 * NT + f) * b.n + m2];   // as bp of interface j-3/2
-      a += i_sl[(long long)(1 * NT + f) * b.n + li];   // middle of its own slope
-      a += i_sl[(long long)(0 * NT + f) * b.n + p1];   // left cell of slope j+1
-      a += i_sl[(long long)(2 * NT + f) * b.n + m1];   // right cell of slope j-1
+      a += i_if[(long long)(1 * NT + f) * b.n + li];  // as a of interface j+1/2
+      a += i_sl[(long long)(1 * NT + f) * b.n + li];  // middle of its own slope
+      if (DIR != 0 || i > 0) {
+        a += i_if[(long long)(2 * NT + f) * b.n + m1];  // as b of interface j-1/2
+        a += i_sl[(long long)(2 * NT + f) * b.n + m1];  // right cell of slope j-1
+      } else {
+        a += i_xif[(2 * NT + f) * np + pen];
+        a += i_xsl[(2 * NT + f) * np + pen];
+      }
+      if (DIR != 0 || i < b.nx - 1) {
+        a += i_if[(long long)(0 * NT + f) * b.n + p1];  // as am of interface j+3/2
+        a += i_sl[(long long)(0 * NT + f) * b.n + p1];  // left cell of slope j+1
+      } else {
+        a += i_xsl[(3 * NT + f) * np + pen];
+      }
+      if (DIR != 0 || i > 1) a += i_if[(long long)(3 * NT + f) * b.n + m2];  // as bp of interface j-3/2
+      else if (i == 1) a += i_xif[(3 * NT + f) * np + pen];
       lt[f] = a;
     }
     Raw9<double> r;
@@ -1100,6 +1169,41 @@ __global__ void k_tvd_t4(Consts c, const Dyn* dyn, Box b, const double* __restri
     double lr[9];  // the cell quantities transposed onto the sweep input
     tvd_cell_rev(c, r, c.kd.hfb[xi], c.kd.hft[xi], s.cmax_t, s.fac0, s.hyper, s.inv_va2max, lt, lr);
     for (int q = 0; q < NV; q++) lam_in[(long long)q * b.n + li] = i_in[(long long)q * b.n + li] + lr[q];
+    lam_p[li] += lr[8];
+  }
+}
+
+// The x sweep's four ghosts of each pencil (-2, -1, nx, nx+1), after k_tvd_t4:
+// their TCell adjoints through the cell quantities, added to the cells they image.
+__global__ void k_tvd_x4(Consts c, const Dyn* dyn, Box b, const double* __restrict__ V, const double* __restrict__ P,
+                         const double* __restrict__ i_if, const double* __restrict__ i_sl,
+                         const double* __restrict__ i_xif, const double* __restrict__ i_xsl,
+                         double* __restrict__ lam_in, double* __restrict__ lam_p) {
+  const Sweep s = sweep_of<0>(c, dyn);
+  const Geom& g = c.g;
+  const int np = b.ny * b.nz;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * np; t += gridDim.x * blockDim.x) {
+    const int e = t / np, pen = t - e * np, j = pen % b.ny, k = pen / b.ny;
+    const int i = e < 2 ? e - 2 : b.nx + e - 2;
+    const long long first = lin(b, 0, j, k), last = lin(b, b.nx - 1, j, k);
+    auto xif = [&](int r, int f) { return i_xif[(long long)(r * NT + f) * np + pen]; };             // interface -1/2
+    auto xsl = [&](int end, int r, int f) { return i_xsl[(long long)((end * 3 + r) * NT + f) * np + pen]; };
+    auto iff = [&](long long l, int r, int f) { return i_if[(long long)(r * NT + f) * b.n + l]; };
+    auto slp = [&](long long l, int r, int f) { return i_sl[(long long)(r * NT + f) * b.n + l]; };
+    double lt[NT];
+    for (int f = 0; f < NT; f++) {
+      if (e == 0) lt[f] = xif(0, f) + xsl(0, 0, f);
+      else if (e == 1) lt[f] = xif(1, f) + iff(first, 0, f) + xsl(0, 1, f) + slp(first, 0, f);
+      else if (e == 2) lt[f] = iff(last, 2, f) + iff(last - 1, 3, f) + xsl(1, 1, f) + slp(last, 2, f);
+      else lt[f] = iff(last, 3, f) + xsl(1, 2, f);
+    }
+    Raw9<double> r;
+    raw_at(g, V, P, fwd(g, i, j, k), r);
+    const int xi = GH + i;
+    double lr[9];
+    tvd_cell_rev(c, r, c.kd.hfb[xi], c.kd.hft[xi], s.cmax_t, s.fac0, s.hyper, s.inv_va2max, lt, lr);
+    const long long li = lin(b, wrap(i, b.nx), j, k);
+    for (int q = 0; q < NV; q++) lam_in[(long long)q * b.n + li] += lr[q];
     lam_p[li] += lr[8];
   }
 }
@@ -1166,9 +1270,15 @@ static void tvd_dir(const Consts& c, const Dyn* dyn, const adj::Box& b, const do
   const int gr = adj_grid(b.n);
   adj::k_tvd_t0<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.tcell);
   adj::k_tvd_t1<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.tcell, lam_out, final_pass, w.in, w.cell, w.fp, w.fm);
+  // the x ghosts, one to four threads per pencil
+  const int np = b.ny * b.nz;
   adj::k_tvd_t2<DIR><<<gr, 128, 0, s>>>(c, dyn, b, w.tcell, w.fp, w.fm, w.iface);
-  adj::k_tvd_t3<DIR><<<gr, 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.slope);
-  adj::k_tvd_t4<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.in, w.cell, w.iface, w.slope, lam_in, lam_p);
+  if (DIR == 0) adj::k_tvd_x2<<<adj_grid(np), 128, 0, s>>>(c, dyn, b, w.tcell, w.fm, w.xif);
+  adj::k_tvd_t3<DIR><<<gr, 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.xif, w.slope);
+  if (DIR == 0) adj::k_tvd_x3<<<adj_grid(2LL * np), 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.xif, w.xsl);
+  adj::k_tvd_t4<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.in, w.cell, w.iface, w.slope, w.xif, w.xsl, lam_in, lam_p);
+  if (DIR == 0)
+    adj::k_tvd_x4<<<adj_grid(4LL * np), 128, 0, s>>>(c, dyn, b, V, P, w.iface, w.slope, w.xif, w.xsl, lam_in, lam_p);
 }
 
 void adjoint_tvd(const Consts& c, const Dyn* dyn, int dir, const double* V, const double* P, const double* lam_out,

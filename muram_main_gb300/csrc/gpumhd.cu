@@ -2371,6 +2371,8 @@ extern "C" int gpumhd_adjoint(gpumhd_ctx* ctx, int nsteps, int checkpoint_every,
   double *bdq = m.get(ctx, 36 * n, &rc), *bwc = m.get(ctx, 11 * n, &rc);
   double* tv = m.get(ctx, (size_t)ADJ_TVD_DOUBLES * n, &rc);
   double* tcell = m.get(ctx, 19 * N, &rc);
+  const size_t np = (size_t)c.g.ny * c.g.nz;
+  double* xg = m.get(ctx, (size_t)ADJ_X_DOUBLES * np, &rc);
   Dyn* adyn = nullptr;
   if (!rc && cudaMalloc(&adyn, sizeof(Dyn)) != cudaSuccess) rc = fail(ctx, GPUMHD_E_NOMEM, "adjoint: Dyn");
   if (rc) { cudaFree(adyn); return rc; }
@@ -2385,6 +2387,8 @@ extern "C" int gpumhd_adjoint(gpumhd_ctx* ctx, int nsteps, int checkpoint_every,
   w.iface = w.fm + 9 * n;
   w.slope = w.iface + 92 * n;
   w.tcell = tcell;
+  w.xif = xg;
+  w.xsl = xg + 92 * np;
   using L = Launch<double>;
   // one recorded forward step: (A, Q0) -> (An, Qn), intermediates kept
   auto record = [&]() {
@@ -2453,7 +2457,7 @@ extern "C" int gpumhd_adjoint(gpumhd_ctx* ctx, int nsteps, int checkpoint_every,
     adjoint_stage(c, adyn, A, Q0, A, lC, lU0, lB, lP, bdq, bwc, 1, s);
     adjoint_eos(c, A, lP, lB, s);
     adjoint_add(c, lB, lU0, lA, s);
-    ctx->launches += 12 + 8 + 5;
+    ctx->launches += 3 * 5 + 3 + 4 * 2 + 4 + 1;  // sweeps, their x ghosts, stages, pressures, sum
     rc = check_launch(ctx, 0);
     if (rc) return rc;
   }

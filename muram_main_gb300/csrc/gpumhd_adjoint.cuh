@@ -16,8 +16,11 @@ struct AdjTvdScratch {
   double* iface;
   double* slope;
   double* tcell;  // the sweep's per-cell TVD quantities, 19 per node of the ghosted box
+  double* xif;    // x sweep, per pencil: interface -1/2 (92) and
+  double* xsl;    // the slopes of cells -1 and nx (2 x 57)
 };
 constexpr int ADJ_TVD_DOUBLES = 8 + 19 + 9 + 9 + 92 + 57;
+constexpr int ADJ_X_DOUBLES = 92 + 2 * 57;
 constexpr int ADJ_STAGE_DOUBLES = 36 + 11;
 
 // Stage `stage` (1..4) with input Uin / Pin (its pressure) and step state U0;

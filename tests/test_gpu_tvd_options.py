@@ -129,3 +129,46 @@ def test_fused_steps_above_the_mach_threshold(gpu_lib):
     e = H.rel_linf(g.download_state(), st.U)
     g.close()
     assert np.all(e <= 1e-12), e
+
+
+def test_adjoint_above_the_mach_threshold(gpu_lib):
+    """The gradient of the top layers' B_x^2 after three steps with tau0 = 0,
+    projected on random directions, against central differences of the forward
+    steps; the field keeps its diffusivity in the fast cells in both."""
+    nx, ny, nz, steps = 16, 12, 8, 3
+    tab = initial.EosTable(H.EOS_SMALL)
+    U0 = initial.periodic_box(tab, nx, ny, nz, seed=41)
+    # diffusivities that depend on the cell's Alfven speed, through the Boris factor
+    kw = dict(tau0=0.0, tvd_h=[2.0, 2.0, 1.0, 2.0], va_max=1.5e5, tvd=list(TVD))
+    kw["tvd"][9] = _mach_threshold(_Oracle(kw, (nx, ny, nz), U0, False))
+    g = gpumhd.MuramGPU(gpumhd.default_params(nx, ny, nz, 3.2e6, **kw), eos_path=H.EOS_SMALL)
+    g.upload_state(U0)
+    dt = 0.6 * float(g.run_steps(1)[0])
+    g.close()
+    g = gpumhd.MuramGPU(gpumhd.default_params(nx, ny, nz, 3.2e6, autostep=0, dt=dt, **kw),
+                        eos_path=H.EOS_SMALL)
+    mask = np.random.default_rng(7).uniform(0.0, 1.0, (nz, ny, 8))
+
+    def after(U):
+        g.upload_state(U)
+        g.run_steps(steps)
+        return g.download_state()
+
+    UT = after(U0)
+    lam = np.zeros_like(UT)
+    lam[5, 2:-2, 2:-2, -10:-2] = 2.0 * mask * UT[5, 2:-2, 2:-2, -10:-2]
+    g.upload_state(U0)
+    grad = g.adjoint(steps, lam, checkpoint_every=2)
+    rng = np.random.default_rng(3)
+    scale = np.sqrt(np.mean(U0[:, 2:-2, 2:-2, 2:-2] ** 2, axis=(1, 2, 3)))
+    errs = []
+    for _ in range(6):
+        v = np.zeros_like(U0)
+        v[:, 2:-2, 2:-2, 2:-2] = rng.standard_normal(U0[:, 2:-2, 2:-2, 2:-2].shape) * scale[:, None, None, None]
+        v = initial.fill_ghosts(v, periodic_x=True)
+        J = [float(np.sum(mask * after(U0 + s * 1e-8 * v)[5, 2:-2, 2:-2, -10:-2] ** 2)) for s in (1, -1)]
+        fd = (J[0] - J[1]) / 2e-8
+        errs.append(abs(float(np.sum(grad * v)) - fd) / abs(fd))
+    g.close()
+    print("adjoint vs central differences, relative errors:", np.array2string(np.array(errs), precision=2))
+    assert np.median(errs) < 1e-6 and max(errs) < 1e-5, errs

@@ -291,6 +291,9 @@ template <class R> __device__ __forceinline__ R mad(const R& a, const R& b, cons
 template <> __device__ __forceinline__ double mad<double>(const double& a, const double& b, const double& c) { return __fma_rn(a, b, c); }
 template <class R> __device__ __forceinline__ R nmad(const R& a, const R& b, const R& c) { return c - a * b; }
 template <> __device__ __forceinline__ double nmad<double>(const double& a, const double& b, const double& c) { return __fma_rn(-a, b, c); }
+// A product that no sum is contracted with.
+__device__ __forceinline__ double mul_apart(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_apart(float a, float b) { return __fmul_rn(a, b); }
 template <class R> __device__ __forceinline__ R dot3(const R& a1, const R& b1, const R& a2, const R& b2, const R& a3, const R& b3) {
   return mad(a3, b3, mad(a2, b2, a1 * b1));
 }

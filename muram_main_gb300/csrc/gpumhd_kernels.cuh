@@ -1600,7 +1600,9 @@ __global__ void __launch_bounds__(256, EwBlocks<R>::v) k_source_integrate(Consts
     if (diag) {
       const R dn = invRdt * u[4];
       diag[3 * N + id] = (dn > (R)0 && dn < (R)INFINITY) ? (R)1.0 : d_div(dn, d_fmax(dn, (R)0.0));
-      diag[4 * N + id] = kc<R>(c).gx * u[0] * u[1];
+      // products of their own: as further uses of the update's they would decide
+      // which of its sums the compiler contracts, and the state would depend on diag
+      diag[4 * N + id] = mul_apart(mul_apart(kc<R>(c).gx, u[0]), u[1]);
       diag[5 * N + id] = b3;
       diag[6 * N + id] += (un[4] - ee) * invdt;
     }

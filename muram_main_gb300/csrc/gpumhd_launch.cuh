@@ -47,8 +47,9 @@ struct Launch {
   // td: cells per thread along the y / z sweeps (0: tvd_chunk's choice; negative: that, but at most -td); the sweeps store the
   // interior (and after a first half pass the periodic images), step_finish
   // then ends the step
-  // dg (per-routine TVDlimit on an output step): the diagnostics, through the
-  // pencil kernel in every direction
+  // dg (per-routine TVDlimit on an output step, never compensated): the
+  // diagnostics; through the pencil kernel in every direction where rho_log = 0
+  // or in FP64
   // Cc (FP32 compensated fused steps, else null): the state's rounding remainders,
   // two arrays of 8N: the current ones, and the x sweep's output
   static void tvd(const Consts& c, int dir, int mode, int only_two_half, const R* Uin, const R* Pst, R* Uout,
@@ -311,12 +312,6 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
   const long long total = (long long)ta.na * ta.nb * nch;
   const int block = 128;
   const long long blocks = (total + block - 1) / block;
-  if (dg) {
-    if (dir == 0) k_tvd_sweep<R, 0, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
-    else if (dir == 1) k_tvd_sweep<R, 1, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
-    else k_tvd_sweep<R, 2, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
-    return;
-  }
   // compensated: the remainders go to the second array in x, back in y, and stay in place in z
   Rem<R>* const C2 = Cc ? Cc + 8 * g.N : nullptr;
   const Rem<R>* const Ci = dir == 1 ? C2 : Cc;
@@ -331,11 +326,23 @@ void Launch<R>::tvd(const Consts& c, int dir, int mode, int only_two_half, const
       // at least one warp per segment (28 cells)
       const long long least = ((g.nx + 27) / 28 + 3) / 4;
       if (nb < least) nb = least;
-      if (dir == 0) (Cc ? k_tvd_xlanes_f32<true> : k_tvd_xlanes_f32<false>)<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Ci, Co);
-      else if (dir == 1) (Cc ? k_tvd_pencil_f32<1, true> : k_tvd_pencil_f32<1, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Ci, Co);
-      else (Cc ? k_tvd_pencil_f32<2, true> : k_tvd_pencil_f32<2, false>)<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Ci, Co);
+      const TvdDiag<R> q = dg ? *dg : TvdDiag<R>{nullptr, (R)0, (R)0};
+      if (dir == 0) {
+        auto* k = dg ? k_tvd_xlanes_f32<false, true> : (Cc ? k_tvd_xlanes_f32<true> : k_tvd_xlanes_f32<false>);
+        k<<<(unsigned)nb, block, 0, s>>>(c, Uin, Pst, Uout, dyn, only_two_half, Ci, Co, q);
+      } else {
+        auto* k = dir == 1 ? (dg ? k_tvd_pencil_f32<1, false, true> : (Cc ? k_tvd_pencil_f32<1, true> : k_tvd_pencil_f32<1, false>))
+                           : (dg ? k_tvd_pencil_f32<2, false, true> : (Cc ? k_tvd_pencil_f32<2, true> : k_tvd_pencil_f32<2, false>));
+        k<<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, Ci, Co, q);
+      }
       return;
     }
+  }
+  if (dg) {
+    if (dir == 0) k_tvd_sweep<R, 0, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
+    else if (dir == 1) k_tvd_sweep<R, 1, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
+    else k_tvd_sweep<R, 2, true><<<(unsigned)blocks, block, 0, s>>>(c, Uin, Pst, Uout, dyn, ta, *dg, nullptr, nullptr);
+    return;
   }
   const TvdDiag<R> nod{nullptr, (R)0, (R)0};
   if (dir == 0) {

@@ -24,8 +24,11 @@
 // 0.69; compensated with 4 spills: 0.39); x 5, 6 (with 6: 0.395; without the
 // prefetch of the next pencil 0.446).
 //
+// DIAG adds an output step's diagnostics (src/tvdlimit_SR.C:577-667) to the same
+// arithmetic, so that asking for them leaves the state's bits alone.
+//
 // k_tvd_sweep<float> and k_tvd_sweep_xlanes<float> stay for runs without the
-// logarithm (rho_log = 0) and for an output step's diagnostics.
+// logarithm (rho_log = 0).
 #pragma once
 
 namespace gpumhd {
@@ -216,12 +219,13 @@ __device__ __forceinline__ float2 limited_diff(float2 d, float2 sa, float2 sb, f
 
 // tvd_flux (src/tvdlimit_SR.C:436-563), times dtt, between cells a (index ia,
 // vertical index xi) and b; dm, dp: the density, velocity and energy differences
-// of the interfaces left of a and right of b (hyperdiffusion).
-template <int DIR>
+// of the interfaces left of a and right of b (hyperdiffusion).  DIAG: qvis
+// receives the viscous heating at the interface.
+template <int DIR, bool DIAG = false>
 __device__ __forceinline__ void flux(const Consts& c, const KC<float>& k, const Cell& a, float b_cm, float b_hd,
                                      const float2 d[4], const float2 sa[4], const float2 sb[4], const float* dm,
                                      const float* dp, int ia, int xi, int sz, int istart, const Sweep& s, float2 F[4],
-                                     float& qres) {
+                                     float& qres, float* qvis = nullptr) {
   F[0] = limited_diff(d[0], sa[0], sb[0], f2(a.he, a.hv));
   F[1] = limited_diff(d[1], sa[1], sb[1], f2(a.hv, a.hv));
   F[2] = limited_diff(d[2], sa[2], sb[2], f2(a.he, a.hB));
@@ -265,13 +269,18 @@ __device__ __forceinline__ void flux(const Consts& c, const KC<float>& k, const 
   F[2].x = f4;
   if (DIR == 0 && !c.g.periodic_x && (ia == sz - GH - 1 || ia == GH - 1)) F[2].y = 0.0f;
   qres = d[2].y * F[2].y + d[3].x * F[3].x + d[3].y * F[3].y;
+  if (DIAG) *qvis = d[0].y * F[0].y + d[1].x * F[1].x + d[1].y * F[1].y;
 }
 
 // tvd_update (src/tvdlimit_SR.C:565-657); Fp / Fm, qp / qm carry the time step.
-// Cin, Cout: the compensated mode's remainders, as in tvd_update.
+// Cin, Cout: the compensated mode's remainders, as in tvd_update.  DIAG: dg, the
+// cell's diagnostics (arrays N apart), per unit of the full step's time; qvp, qvm:
+// the viscous heating at the cell's interfaces, times dtt.
+template <bool DIAG = false>
 __device__ __forceinline__ void update(const KC<float>& k, const float2 Fp[4], const float2 Fm[4], float qp, float qm,
                                        const Cell& c0, const float* u_in, float* u, const Rem<float>* Cin,
-                                       Rem<float>* Cout, long long N) {
+                                       Rem<float>* Cout, long long N, float* dg = nullptr, float idt = 0.0f,
+                                       float qvp = 0.0f, float qvm = 0.0f) {
   float res[NV];
 #pragma unroll
   for (int p = 0; p < 4; p++) {
@@ -280,12 +289,18 @@ __device__ __forceinline__ void update(const KC<float>& k, const float2 Fp[4], c
     res[2 * p + 1] = r.y;
   }
   const float v1 = c0.q[0].y, v2 = c0.q[1].x, v3 = c0.q[1].y, b1 = c0.q[2].y, b2 = c0.q[3].x, b3 = c0.q[3].y;
+  if (DIAG) {
+    dg[7 * N] += (res[4] + (1.0f - c0.qt) * (res[1] * v1 + res[2] * v2 + res[3] * v3)) * idt;
+    dg[8 * N] += 0.5f * (qp + qm) * c0.qt * idt;
+    dg[9 * N] += 0.5f * (qvp + qvm) * c0.qt * idt;
+  }
   res[4] += (1.0f - c0.qt) * (res[1] * v1 + res[2] * v2 + res[3] * v3) + 0.5f * (qp + qm) * c0.qt;
   const float dn = (res[1] * b1 + res[2] * b2 + res[3] * b3) * rcp(fmaxf(1e-30f, c0.bsqr));
   const float g1 = c0.BC2 * (dn * b1 - res[1]), g2 = c0.BC2 * (dn * b2 - res[2]), g3 = c0.BC2 * (dn * b3 - res[3]);
   res[1] += g1;
   res[2] += g2;
   res[3] += g3;
+  if (DIAG) dg[5 * N] += (g1 * v1 + g2 * v2 + g3 * v3) * idt;
   res[4] += g1 * v1 + g2 * v2 + g3 * v3;
   float rem[NV];
   if (Cin) {
@@ -302,6 +317,7 @@ __device__ __forceinline__ void update(const KC<float>& k, const float2 Fp[4], c
   const float d0 = u[0], e0 = u[4];
   u[0] = fmaxf(k.rho_min, d0);
   u[4] = fmaxf(e0, k.eps_min * u[0] + 0.5f * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) * rcp(u[0]));
+  if (DIAG) dg[6 * N] += (u[4] - e0) * idt;
   if (Cin && Cout) {
     if (u[0] != d0) rem[0] = 0.0f;
     if (u[4] != e0) rem[4] = 0.0f;
@@ -318,11 +334,11 @@ __device__ __forceinline__ Sweep sweep_of(const DynR<float>& dr, const KC<float>
 
 // Sweep along y (DIR 1) or z (DIR 2): one thread per pencil chunk, marching with
 // a window of cells; the next cell's stored values are loaded a step ahead.
-template <int DIR, bool COMP>
-__global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, const float* __restrict__ Uin,
+template <int DIR, bool COMP, bool DIAG = false>
+__global__ void __launch_bounds__(128, COMP || DIAG ? 3 : 4) k_tvd_pencil_f32(Consts c, const float* __restrict__ Uin,
                                                            const float* __restrict__ Pst, float* __restrict__ Uout,
                                                            Dyn* __restrict__ dyn, TvdArgs ta,
-                                                           const Rem<float>* Ci, Rem<float>* Co) {
+                                                           const Rem<float>* Ci, Rem<float>* Co, TvdDiag<float> dg) {
   using namespace tvdf;
   if (dyn->err) return;
   if (ta.only_two_half && !dyn->two_half) return;  // second half pass not taken this step
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
   const Prof pr = prof_of(k, aa);
   Cell c0, c1;
   float2 d0[4], s0[4], F0[4];
-  float q0;
+  float q0, qv0 = 0.0f;  // qv: viscous heating, for the diagnostics
   Raw9<float> nxt;
   unsigned off = base + (unsigned)p0 * sd;
   {
@@ -365,19 +381,19 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
     load9(Uin, Pst, N, off + 2u * sd, nxt);
     diff(c0, c1, d0);
     slope(k, db, d0, c0.vsqr, s.vsqr_diff, aa, s0);
-    flux<DIR>(c, k, cb, c0.cm, 0.0f, db, sm, s0, nullptr, nullptr, p0 - 1, aa, 0, 0, s, F0, q0);
+    flux<DIR, DIAG>(c, k, cb, c0.cm, 0.0f, db, sm, s0, nullptr, nullptr, p0 - 1, aa, 0, 0, s, F0, q0, &qv0);
   }
   // one cell: window a | b | n (n read from nxt), interface a | b with differences
   // da and slopes sa, sb; the values a later cell needs go to n, dn, sb, F, q
   auto step = [&](int pos, const Cell& a, const Cell& b, Cell& n, const float2* da, float2* db, const float2* sa,
-                  float2* sb, const float2* Fm, float2* F, float qm, float& q) {
+                  float2* sb, const float2* Fm, float2* F, float qm, float& q, float qvm, float& qv) {
     float uc[NV], u[NV];
     load8(Uin, N, off, uc);
     cell_of(k, nxt, pr, s, n);
     if (pos + 1 < p1) load9(Uin, Pst, N, off + 3u * sd, nxt);
     diff(b, n, db);
     slope(k, da, db, b.vsqr, s.vsqr_diff, aa, sb);
-    flux<DIR>(c, k, a, b.cm, 0.0f, da, sa, sb, nullptr, nullptr, pos, aa, 0, 0, s, F, q);
+    flux<DIR, DIAG>(c, k, a, b.cm, 0.0f, da, sa, sb, nullptr, nullptr, pos, aa, 0, 0, s, F, q, &qv);
     const int cj = DIR == 1 ? pos : bb, ck = DIR == 2 ? pos : bb;
     const Rem<float>* cin = nullptr;
     Rem<float>* cout = nullptr;
@@ -386,7 +402,7 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
       cin = Ci + cidx32(g, aa, sj, sk);
       if (sj == cj && sk == ck) cout = Co + cidx32(g, aa, cj, ck);
     }
-    update(k, F, Fm, q, qm, a, uc, u, cin, cout, N);
+    update<DIAG>(k, F, Fm, q, qm, a, uc, u, cin, cout, N, DIAG ? dg.d + off / 4u : nullptr, dg.idt_full, qv, qvm);
     if (!half_images) store8(Uout, N, off, u);
     else store_state<float, true>(g, Uout, aa, cj, ck, images_of(g, aa, cj, ck, false), u);
     off += sd;
@@ -395,10 +411,10 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
   for (int pos = p0; pos < p1; pos += 2) {
     Cell c2;
     float2 d1[4], s1[4], F1[4];
-    float q1;
-    step(pos, c0, c1, c2, d0, d1, s0, s1, F0, F1, q0, q1);
+    float q1, qv1 = 0.0f;
+    step(pos, c0, c1, c2, d0, d1, s0, s1, F0, F1, q0, q1, qv0, qv1);
     if (pos + 1 >= p1) break;
-    step(pos + 1, c1, c2, c0, d1, d0, s1, s0, F1, F0, q1, q0);
+    step(pos + 1, c1, c2, c0, d1, d0, s1, s0, F1, F0, q1, q0, qv1, qv0);
     c1 = c0;
     c0 = c2;
   }
@@ -407,11 +423,11 @@ __global__ void __launch_bounds__(128, COMP ? 3 : 4) k_tvd_pencil_f32(Consts c, 
 // Sweep along x: 32 consecutive cells of a pencil per warp, one per lane; the
 // two lanes at each end are the stencil's halo (28 updates per warp), as in
 // k_tvd_sweep_xlanes.
-template <bool COMP>
+template <bool COMP, bool DIAG = false>
 __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, const float* __restrict__ Uin,
                                                            const float* __restrict__ Pst, float* __restrict__ Uout,
                                                            Dyn* __restrict__ dyn, int only_two_half,
-                                                           const Rem<float>* Ci, Rem<float>* Co) {
+                                                           const Rem<float>* Ci, Rem<float>* Co, TvdDiag<float> dg) {
   using namespace tvdf;
   if (dyn->err) return;
   if (only_two_half && !dyn->two_half) return;
@@ -466,11 +482,12 @@ __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, 
       dp[1] = __shfl_down_sync(ALL, dr[0].y, 1);
       dp[2] = __shfl_down_sync(ALL, dr[2].x, 1);
     }
-    float q;
-    flux<0>(c, k, c0, r_cm, r_hd, dr, s0, s1, dm, dp, pos, posc, g.nx + 2 * GH, istart, s, F, q);
+    float q, qv = 0.0f;
+    flux<0, DIAG>(c, k, c0, r_cm, r_hd, dr, s0, s1, dm, dp, pos, posc, g.nx + 2 * GH, istart, s, F, q, &qv);
 #pragma unroll
     for (int p = 0; p < 4; p++) Fm[p] = up1(F[p]);
     const float qm = __shfl_up_sync(ALL, q, 1);
+    const float qvm = DIAG ? __shfl_up_sync(ALL, qv, 1) : 0.0f;
     if (!out) continue;
     const unsigned id = base + (unsigned)pos;
     const Rem<float>* cin = nullptr;
@@ -482,7 +499,7 @@ __global__ void __launch_bounds__(128, COMP ? 6 : 5) k_tvd_xlanes_f32(Consts c, 
       if (sj == j && sk == kz) cout = Co + id;
     }
     float u[NV];
-    update(k, F, Fm, q, qm, c0, uin, u, cin, cout, g.N);
+    update<DIAG>(k, F, Fm, q, qm, c0, uin, u, cin, cout, g.N, DIAG ? dg.d + id : nullptr, dg.idt_full, qv, qvm);
     store8(Uout, g.N, id * 4u, u);
   }
 }

@@ -395,12 +395,18 @@ struct C2POut {
   double pres, temp, ne, rhoi, amb;
 };
 
-// Full ConsToPrim arithmetic for one cell given primitives (src/cons_to_prim.C:148-243).
-__device__ inline C2POut c2p_eos_full(const Consts& c, double d, double ei, double dn) {
-  const double eps = mad(ei, dn, c.eps_off);
-  const double lgr = d_log(d);
-  const double ep = d_log(eps);
-  const double lr = lgr;
+// A cell's place in the EOS tables (src/cons_to_prim.C:148-175): offsets and
+// weights of the bilinear sum.
+struct EosCell {
+  double eps, lgr;
+  double w[4];
+  long long a[4];
+};
+__device__ inline EosCell eos_cell(const Consts& c, double d, double ei, double dn) {
+  EosCell q;
+  q.eps = mad(ei, dn, c.eps_off);
+  q.lgr = d_log(d);
+  const double ep = d_log(q.eps), lr = q.lgr;
   // (int) as x86-64 does it, then at least 0: out of range and NaN give 0
   int i_d = i64f::trunc_pos((lr - c.xlr0) * c.inv_del_lr);
   i_d = min(c.N_lr - 2, i_d);
@@ -408,25 +414,31 @@ __device__ inline C2POut c2p_eos_full(const Consts& c, double d, double ei, doub
   i_e = min(c.N_eps - 2, i_e);
   const double xe0 = c.xeps[i_e], xe1 = c.xeps[i_e + 1];
   const double xr0 = c.xlr[i_d], xr1 = c.xlr[i_d + 1];
-  const double c0 = (ep - xe0) * (lr - xr0);
-  const double c1 = (ep - xe0) * (xr1 - lr);
-  const double c2 = (xe1 - ep) * (lr - xr0);
-  const double c3 = (xe1 - ep) * (xr1 - lr);
-  const long long a11 = (long long)(i_e + 1) * c.N_lr + (i_d + 1);
-  const long long a10 = (long long)(i_e + 1) * c.N_lr + i_d;
-  const long long a01 = (long long)i_e * c.N_lr + (i_d + 1);
-  const long long a00 = (long long)i_e * c.N_lr + i_d;
+  q.w[0] = (ep - xe0) * (lr - xr0);
+  q.w[1] = (ep - xe0) * (xr1 - lr);
+  q.w[2] = (xe1 - ep) * (lr - xr0);
+  q.w[3] = (xe1 - ep) * (xr1 - lr);
+  q.a[0] = (long long)(i_e + 1) * c.N_lr + (i_d + 1);
+  q.a[1] = (long long)(i_e + 1) * c.N_lr + i_d;
+  q.a[2] = (long long)i_e * c.N_lr + (i_d + 1);
+  q.a[3] = (long long)i_e * c.N_lr + i_d;
+  return q;
+}
+// exp of the bilinear sum of table T
+__device__ inline double eos_value(const EosCell& q, const float* T) {
+  double s = q.w[0] * i64f::from_float(T[q.a[0]]);
+#pragma unroll
+  for (int k = 1; k < 4; k++) s = mad(q.w[k], i64f::from_float(T[q.a[k]]), s);
+  return d_exp(s);
+}
+
+// Full ConsToPrim arithmetic for one cell given primitives (src/cons_to_prim.C:148-243).
+__device__ inline C2POut c2p_eos_full(const Consts& c, double d, double ei, double dn) {
+  const EosCell q = eos_cell(c, d, ei, dn);
+  const double eps = q.eps, lgr = q.lgr;
   double out[6];
 #pragma unroll
-  for (int t = 0; t < 6; t++) {
-    if (t == 2) { out[t] = 0.0; continue; }
-    const float* T = c.tab[t];
-    double s = c0 * i64f::from_float(T[a11]);
-    s = mad(c1, i64f::from_float(T[a10]), s);
-    s = mad(c2, i64f::from_float(T[a01]), s);
-    s = mad(c3, i64f::from_float(T[a00]), s);
-    out[t] = d_exp(s);
-  }
+  for (int t = 0; t < 6; t++) out[t] = t == 2 ? 0.0 : eos_value(q, c.tab[t]);
   double pr = out[0], tm = out[1], nl = out[3];
   if (lgr < c.xlr0) {
     pr = c.c_pres * ei;

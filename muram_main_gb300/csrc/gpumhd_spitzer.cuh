@@ -30,37 +30,9 @@ template <> __device__ __forceinline__ float spt_bbmin<float>() { return 1e-30f;
 // ConsToPrim's temperature (src/cons_to_prim.C:148-243), with the pressure its
 // fallback tests: c2p_eos_full's arithmetic for those two outputs.
 __device__ inline double c2p_temp(const Consts& c, double d, double ei, double dn) {
-  const double eps = ei * dn + c.eps_off;
-  const double lgr = log(d);
-  const double ep = log(eps);
-  const double lr = lgr;
-  int i_d = cvt_x86((lr - c.xlr0) * c.inv_del_lr);
-  i_d = max(0, i_d);
-  i_d = min(c.N_lr - 2, i_d);
-  int i_e = cvt_x86((ep - c.xeps0) * c.inv_del_eps);
-  i_e = max(0, i_e);
-  i_e = min(c.N_eps - 2, i_e);
-  const double xe0 = c.xeps[i_e], xe1 = c.xeps[i_e + 1];
-  const double xr0 = c.xlr[i_d], xr1 = c.xlr[i_d + 1];
-  const double c0 = (ep - xe0) * (lr - xr0);
-  const double c1 = (ep - xe0) * (xr1 - lr);
-  const double c2 = (xe1 - ep) * (lr - xr0);
-  const double c3 = (xe1 - ep) * (xr1 - lr);
-  const long long a11 = (long long)(i_e + 1) * c.N_lr + (i_d + 1);
-  const long long a10 = (long long)(i_e + 1) * c.N_lr + i_d;
-  const long long a01 = (long long)i_e * c.N_lr + (i_d + 1);
-  const long long a00 = (long long)i_e * c.N_lr + i_d;
-  double out[2];
-#pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const float* T = c.tab[t];
-    double s = c0 * (double)T[a11];
-    s += c1 * (double)T[a10];
-    s += c2 * (double)T[a01];
-    s += c3 * (double)T[a00];
-    out[t] = exp(s);
-  }
-  double pr = out[0], tm = out[1];
+  const EosCell q = eos_cell(c, d, ei, dn);
+  const double eps = q.eps, lgr = q.lgr;
+  double pr = eos_value(q, c.tab[0]), tm = eos_value(q, c.tab[1]);
   if (lgr < c.xlr0) {
     pr = c.c_pres * ei;
     tm = c.c_temp * eps;
@@ -103,7 +75,7 @@ __device__ __forceinline__ float eos_temp(const Consts& c, float d, float ei, fl
   return expf(s);
 }
 __device__ __forceinline__ float temp_of(const Consts& c, float d, float ei) { return eos_temp(c, d, ei, 1.0f / d); }
-__device__ __forceinline__ double temp_of(const Consts& c, double d, double ei) { return c2p_temp(c, d, ei, 1.0 / d); }
+__device__ __forceinline__ double temp_of(const Consts& c, double d, double ei) { return c2p_temp(c, d, ei, d_div(1.0, d)); }
 
 // Temperature of every cell, ghosts included, of a conserved state.
 template <class R>

@@ -9,7 +9,12 @@ pytestmark = pytest.mark.gpu
 
 BOXES = [((24, 16, 16), False, {}), ((29, 9, 33), True, {}), ((64, 40, 36), True, {}),
          ((24, 16, 16), False, dict(CFL_tvd=0.3)), ((29, 9, 33), True, dict(eta=1e10)),
-         ((16, 12, 8), False, dict(spitzer=0.5))]
+         ((16, 12, 8), False, dict(spitzer=0.5)),
+         ((24, 16, 16), False, dict(divB_switch=1, divB_itmax=4, divB_err=0.2)),
+         ((24, 16, 16), False, dict(va_adjust=1.0)),
+         ((30, 9, 33), True, dict(xbnd=1, bnd_bcrit=1e3, bnd_eps_top=0.0)),
+         ((30, 9, 33), True, dict(xbnd=1, bnd_bcrit=1e3, bnd_eps_top=0.0, spitzer=0.5, divB_switch=1, divB_itmax=4,
+                                  divB_err=0.2))]
 
 
 def _box(shape, closed, precision, kw):

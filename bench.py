@@ -407,7 +407,7 @@ def run_ours(args):
                 "peak_source": f"{peak_src} hbm_gbs"}
     if dom == "stage":
         roofline["limiter"] = ("instruction issue and dependency latency, not HBM (ncu: ~50 % issue active, "
-                               "24-39 % DRAM throughput)")
+                               "DRAM 2.2-3.5 TB/s, 33-52 % of the measured copy rate)")
     # whole-step bytes against HBM
     step_bytes = ALGO_STEP_WORDS * 4 * n_cells
     step_ms = ms / args.steps

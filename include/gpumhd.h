@@ -120,7 +120,10 @@ int gpumhd_eos_init(gpumhd_ctx* ctx, const char* path);
  * which = 3..7: pres, temp, ne, rhoi, amb; 8: phi, 9: divB (the divB cleaning's
  * potential and last divergence, GridData::phi / divB); 10: sflx (the Spitzer
  * heat flux, GridData::sflx); 11..20: the diagnostics tvar1..tvar8, Qres, Qvis
- * (GridData, see gpumhd_set_need_diagnostics); one double per node. */
+ * (GridData, see gpumhd_set_need_diagnostics); one double per node.  A download
+ * waits for the result.  An upload from pinned host memory is enqueued on the
+ * context's stream: the buffer must stay unchanged until a call that waits
+ * (gpumhd_synchronize, a download); pageable memory may be reused at once. */
 int gpumhd_upload(gpumhd_ctx* ctx, int which, const double* host);
 int gpumhd_download(gpumhd_ctx* ctx, int which, double* host);
 /* The same with float host arrays: the cState arrays (U, U0) of GridData in
@@ -335,9 +338,9 @@ long long gpumhd_ensemble_launch_count(gpumhd_ensemble* e);
  * results do not depend on the schedule. */
 int gpumhd_ensemble_set_schedule(gpumhd_ensemble* e, int steps_per_iteration, int largest_first);
 /* Launch shapes of the boxes for running inside the ensemble: each box's
- * current shapes, or stage z chunks of half or all of its z extent with TVD
- * chunks of 64 or 128 cells (longer marches pay when the other boxes fill the
- * GPU), timed over trial_steps steps of the ensemble from the boxes' current
+ * current shapes, or stage z chunks of a half or a quarter of its z extent with
+ * TVD chunks of 16, 64 or 128 cells (longer marches pay when the other boxes fill
+ * the GPU), timed over trial_steps steps of the ensemble from the boxes' current
  * states and restored states afterwards (state, pressure, divB potential,
  * heat flux, step control); keeps the fastest, branches largest box first.
  * *best_ms: its time per ensemble step. */

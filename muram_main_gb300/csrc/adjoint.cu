@@ -5,12 +5,12 @@
 // with TCheck).  Its adjoint runs the same pieces backwards.  The stencil
 // structure -- which cell's output depends on which neighbours, the transposes
 // of the fourth-order differences and of the TVD interface fluxes -- is
-// written out here; the Jacobians of the cell-local functions (fluxes,
-// residual assembly, sources, Tcheck, EOS pressure, the TVD cell quantities,
-// slopes, interface flux and update) come from forward-mode dual numbers run
-// through the same templates the forward kernels use, so both always agree.
-// Limiter kinks and clamps take the derivative of the branch the forward step
-// took (one-sided subgradients).
+// written out here; the cell-local functions (fluxes, primitives, residual
+// assembly, sources, Boris factor, the TVD cell quantities, slopes, interface
+// flux and update) are transposed in reverse passes that recompute the forward
+// values, and Tcheck and the EOS pressure through forward-mode dual numbers run
+// through the forward's templates.  Limiter kinks and clamps take the derivative
+// of the branch the forward step took (one-sided subgradients).
 //
 // Adjoint fields live on the interior only (nx*ny*nz per variable, x fastest)
 // with periodic neighbours; forward fields are the ghost-filled arrays the

@@ -2168,9 +2168,10 @@ extern "C" int gpumhd_ensemble_set_schedule(gpumhd_ensemble* e, int steps_per_it
 // stencil halo); inside an ensemble the other boxes fill it, so longer
 // marches can pay.  Candidates: each box's current shapes, and stage z chunks
 // of a half or a quarter of the box's z extent with TVD chunks of 16, 64 or 128
-// cells (20 steps of 16 boxes of 32 to 96 cells a side: 21.9 ms with the boxes'
-// own shapes, 20.2 with quarters and 16; 24.3 with halves and 128, which is the
-// fastest for 64 boxes of up to 128 a side; the whole z extent 28 and more);
+// cells (20 steps of 16 boxes of 32 to 96 cells a side: 18.3 ms with the boxes'
+// own shapes, 14.8 with halves and 16, 15.3 with quarters and 16, 16.1 with halves
+// and 64; 17.1 with halves and 128, which is the fastest for 64 boxes of up to 128
+// a side; the whole z extent 23);
 // timed over trial_steps steps of the whole ensemble (branches largest box
 // first) from the boxes' current states, which are restored afterwards.
 extern "C" int gpumhd_ensemble_autotune(gpumhd_ensemble* e, int trial_steps, double* best_ms) {

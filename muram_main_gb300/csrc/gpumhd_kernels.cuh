@@ -1715,7 +1715,9 @@ __global__ void k_fill_ghosts(Geom g, R* __restrict__ U, int nfield, int with_bc
 // A may be device memory (a staging buffer) or pinned host memory, which the
 // kernel then reads or writes over the link itself: the conversion costs no pass
 // of its own (0.64 GB: 3.02 ms up and 3.30 down, as the copies alone take, against
-// 0.2 to 0.3 ms more through a staging buffer).  The link is busy with 38 blocks.
+// 0.2 to 0.3 ms more through a staging buffer), with a grid of at most 304 blocks,
+// two per SM.  Unaligned records (not VEC) come from a staging buffer, but for
+// uploads of floats (gpumhd_hostmem.cuh has both sides' times).
 // VEC: A is 16-byte aligned and nf is 8, so records move in 16-byte pieces;
 // downwards the lanes of a warp exchange values so that each of its stores
 // covers 512 contiguous bytes (one record per thread instead: 8 ms).

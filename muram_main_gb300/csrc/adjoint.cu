@@ -1010,9 +1010,9 @@ __global__ void k_tvd_t1(Consts c, const Dyn* dyn, Box b, const double* __restri
 // a periodic box carry the boundary's values (hb or ht = 1), so the interface at
 // -1/2 is not the image of the one at nx-1/2, nor a ghost's slope and cell
 // quantities those of the cell it images.  In the x sweep each is transposed for
-// itself: interface -1/2 (k_tvd_x2), the slopes of cells -1 and nx (k_tvd_x3) and
-// the cell quantities of the four ghosts (k_tvd_x4), one thread per pencil; y and
-// z sweeps wrap.
+// itself: interface -1/2 by threads of k_tvd_t2 past the cells, the slopes of cells
+// -1 and nx by such threads of k_tvd_t3, and the cell quantities of the four ghosts
+// by k_tvd_x4; y and z sweeps wrap.
 
 // The flux of the interface between T[1] and T[2] (memory index p of T[1])
 // transposed in one reverse pass onto its four cells' TCells (am, a, b, bp: 19
@@ -1050,77 +1050,58 @@ __device__ __forceinline__ void slope_rev(const Consts& c, const Sweep& s, const
 // T2: per interface i+1/2 (stored at its left cell i), the interface flux
 // transposed onto its four cells' TCells (am, a, b, bp: 19 each) and its two
 // slopes (8 each): 92 values per interface.
+// x sweep: interface -1/2 of each pencil to o_xif.
 template <int DIR>
 __global__ void k_tvd_t2(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
-                         const double* __restrict__ i_fp, const double* __restrict__ i_fm, double* __restrict__ o_if) {
+                         const double* __restrict__ i_fp, const double* __restrict__ i_fm, double* __restrict__ o_if,
+                         double* __restrict__ o_xif) {
   const Sweep s = sweep_of<DIR>(c, dyn);
-  for (long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x; li < b.n;
-       li += (long long)gridDim.x * blockDim.x) {
+  const long long np = (long long)b.ny * b.nz, n = DIR == 0 ? b.n + np : b.n;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const bool ghost = DIR == 0 && t >= b.n;
     int i, j, k;
-    ijk(b, li, i, j, k);
-    const long long lr = nbr<DIR>(b, i, j, k, 1);
+    ijk(b, ghost ? (t - b.n) * b.nx : t, i, j, k);
+    const long long lr = ghost ? lin(b, 0, j, k) : nbr<DIR>(b, i, j, k, 1);
+    if (ghost) i = -1;
     const bool last_x = DIR == 0 && i == b.nx - 1;  // cell 0's left flux is interface -1/2's
     double lF[NV + 1];
     for (int q = 0; q <= NV; q++)
-      lF[q] = i_fp[(long long)q * b.n + li] + (last_x ? 0.0 : i_fm[(long long)q * b.n + lr]);
+      lF[q] = (ghost ? 0.0 : i_fp[(long long)q * b.n + t]) + (last_x ? 0.0 : i_fm[(long long)q * b.n + lr]);
     TCell<double> T[4];
     for (int o = -1; o <= 2; o++) cell_load<DIR>(c.g, tc, i, j, k, o, T[o + 1]);
-    interface_rev<DIR>(c, s, T, pos_of<DIR>(i, j, k), lF, o_if + li, b.n);
-  }
-}
-// Interface -1/2 of the x sweep: 92 values per pencil.
-__global__ void k_tvd_x2(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
-                         const double* __restrict__ i_fm, double* __restrict__ o_xif) {
-  const Sweep s = sweep_of<0>(c, dyn);
-  const int np = b.ny * b.nz;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np; t += gridDim.x * blockDim.x) {
-    const int j = t % b.ny, k = t / b.ny;
-    const long long li = lin(b, 0, j, k);
-    double lF[NV + 1];
-    for (int q = 0; q <= NV; q++) lF[q] = i_fm[(long long)q * b.n + li];
-    TCell<double> T[4];
-    for (int o = -1; o <= 2; o++) cell_load<0>(c.g, tc, -1, j, k, o, T[o + 1]);
-    interface_rev<0>(c, s, T, pos_of<0>(-1, j, k), lF, o_xif + t, np);
+    interface_rev<DIR>(c, s, T, pos_of<DIR>(i, j, k), lF, ghost ? o_xif + (t - b.n) : o_if + t, ghost ? np : b.n);
   }
 }
 
 // T3: per cell i, its slope transposed onto the three cells it reads
 // (i-1: q; i: q, hb, ht, vsqr; i+1: q): 3 x 19 values.
+// x sweep: the slopes of cells -1 and nx of each pencil to o_xsl (2 x 57).
 template <int DIR>
 __global__ void k_tvd_t3(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
-                         const double* __restrict__ i_if, const double* __restrict__ i_xif, double* __restrict__ o_sl) {
+                         const double* __restrict__ i_if, const double* __restrict__ i_xif, double* __restrict__ o_sl,
+                         double* __restrict__ o_xsl) {
   const Sweep s = sweep_of<DIR>(c, dyn);
-  const long long np = (long long)b.ny * b.nz;
-  for (long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x; li < b.n;
-       li += (long long)gridDim.x * blockDim.x) {
+  const long long np = (long long)b.ny * b.nz, n = DIR == 0 ? b.n + 2 * np : b.n;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const long long e = DIR == 0 && t >= b.n ? (t - b.n) / np : -1;  // 0: cell -1, 1: cell nx
+    const long long pen = e < 0 ? 0 : t - b.n - e * np;
     int i, j, k;
-    ijk(b, li, i, j, k);
-    const long long ll = nbr<DIR>(b, i, j, k, -1);
-    const bool first_x = DIR == 0 && i == 0;
-    const double* const lb = first_x ? i_xif + (j + (long long)b.ny * k) : i_if + ll;  // the interface left of i
-    const long long sb = first_x ? np : b.n;
+    ijk(b, e < 0 ? t : pen * b.nx, i, j, k);
+    if (e >= 0) i = e == 0 ? -1 : b.nx;
+    const bool left_x = DIR == 0 && i <= 0;  // the interface left of cell 0, right of cell -1
+    const double* const x = i_xif + (j + (long long)b.ny * k);
     double ls[NV];
-    for (int q = 0; q < NV; q++) ls[q] = i_if[(long long)(4 * NT + q) * b.n + li] + lb[(4 * NT + NV + q) * sb];
+    for (int q = 0; q < NV; q++) {
+      const int fa = 4 * NT + q, fb = 4 * NT + NV + q;  // as the interface's left, right cell
+      double l = 0.0;
+      if (e < 0) l += i_if[(long long)fa * b.n + t];
+      else if (e == 0) l += x[fa * np];
+      if (e != 0) l += left_x ? x[fb * np] : i_if[(long long)fb * b.n + (e < 0 ? nbr<DIR>(b, i, j, k, -1) : lin(b, b.nx - 1, j, k))];
+      ls[q] = l;
+    }
     TCell<double> T[3];
     for (int o = -1; o <= 1; o++) cell_load<DIR>(c.g, tc, i, j, k, o, T[o + 1]);
-    slope_rev(c, s, T, ls, o_sl + li, b.n);
-  }
-}
-// The slopes of cells -1 and nx of the x sweep: 2 x 57 values per pencil.
-__global__ void k_tvd_x3(Consts c, const Dyn* dyn, Box b, const double* __restrict__ tc,
-                         const double* __restrict__ i_if, const double* __restrict__ i_xif,
-                         double* __restrict__ o_xsl) {
-  const Sweep s = sweep_of<0>(c, dyn);
-  const int np = b.ny * b.nz;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * np; t += gridDim.x * blockDim.x) {
-    const int end = t / np, pen = t - end * np, j = pen % b.ny, k = pen / b.ny;
-    const long long last = lin(b, b.nx - 1, j, k);
-    double ls[NV];
-    for (int q = 0; q < NV; q++)
-      ls[q] = end == 0 ? i_xif[(long long)(4 * NT + q) * np + pen] : i_if[(long long)(4 * NT + NV + q) * b.n + last];
-    TCell<double> T[3];
-    for (int o = -1; o <= 1; o++) cell_load<0>(c.g, tc, end == 0 ? -1 : b.nx, j, k, o, T[o + 1]);
-    slope_rev(c, s, T, ls, o_xsl + (long long)end * 3 * NT * np + pen, np);
+    slope_rev(c, s, T, ls, e < 0 ? o_sl + t : o_xsl + e * 3 * NT * np + pen, e < 0 ? b.n : np);
   }
 }
 
@@ -1270,15 +1251,12 @@ static void tvd_dir(const Consts& c, const Dyn* dyn, const adj::Box& b, const do
   const int gr = adj_grid(b.n);
   adj::k_tvd_t0<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.tcell);
   adj::k_tvd_t1<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.tcell, lam_out, final_pass, w.in, w.cell, w.fp, w.fm);
-  // the x ghosts, one to four threads per pencil
-  const int np = b.ny * b.nz;
-  adj::k_tvd_t2<DIR><<<gr, 128, 0, s>>>(c, dyn, b, w.tcell, w.fp, w.fm, w.iface);
-  if (DIR == 0) adj::k_tvd_x2<<<adj_grid(np), 128, 0, s>>>(c, dyn, b, w.tcell, w.fm, w.xif);
-  adj::k_tvd_t3<DIR><<<gr, 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.xif, w.slope);
-  if (DIR == 0) adj::k_tvd_x3<<<adj_grid(2LL * np), 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.xif, w.xsl);
+  const long long np = (long long)b.ny * b.nz, x = DIR == 0 ? np : 0;  // the x sweep's ghosts
+  adj::k_tvd_t2<DIR><<<adj_grid(b.n + x), 128, 0, s>>>(c, dyn, b, w.tcell, w.fp, w.fm, w.iface, w.xif);
+  adj::k_tvd_t3<DIR><<<adj_grid(b.n + 2 * x), 128, 0, s>>>(c, dyn, b, w.tcell, w.iface, w.xif, w.slope, w.xsl);
   adj::k_tvd_t4<DIR><<<gr, 128, 0, s>>>(c, dyn, b, V, P, w.in, w.cell, w.iface, w.slope, w.xif, w.xsl, lam_in, lam_p);
   if (DIR == 0)
-    adj::k_tvd_x4<<<adj_grid(4LL * np), 128, 0, s>>>(c, dyn, b, V, P, w.iface, w.slope, w.xif, w.xsl, lam_in, lam_p);
+    adj::k_tvd_x4<<<adj_grid(4 * np), 128, 0, s>>>(c, dyn, b, V, P, w.iface, w.slope, w.xif, w.xsl, lam_in, lam_p);
 }
 
 void adjoint_tvd(const Consts& c, const Dyn* dyn, int dir, const double* V, const double* P, const double* lam_out,

@@ -2458,7 +2458,7 @@ extern "C" int gpumhd_adjoint(gpumhd_ctx* ctx, int nsteps, int checkpoint_every,
     adjoint_stage(c, adyn, A, Q0, A, lC, lU0, lB, lP, bdq, bwc, 1, s);
     adjoint_eos(c, A, lP, lB, s);
     adjoint_add(c, lB, lU0, lA, s);
-    ctx->launches += 3 * 5 + 3 + 4 * 2 + 4 + 1;  // sweeps, their x ghosts, stages, pressures, sum
+    ctx->launches += 3 * 5 + 1 + 4 * 2 + 4 + 1;  // sweeps, their x ghosts, stages, pressures, sum
     rc = check_launch(ctx, 0);
     if (rc) return rc;
   }
